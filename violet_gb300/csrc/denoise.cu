@@ -437,10 +437,7 @@ struct AtrousTaps {
 // svgf_atrous_filter.hlsl:23-88: 5x5 taps at step 2^i, kernel {1, 2/3, 1/6}, only
 // the 16 taps off both centre axes (the shader's `(x != 0) && (y != 0)`).
 template <class Geo>
-struct DnAtrousF {
-  static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, AtrousTaps taps, const uint2* __restrict__ color, const uint32_t* __restrict__ var_tex, uint2* __restrict__ out_color, uint32_t* __restrict__ out_var, uint32_t* __restrict__ out_diff, uint32_t* __restrict__ out_spec, int step) {
-  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
-  if (!inb(x, y, w, h)) return;
+__device__ __forceinline__ void atrous_px(int x, int y, int w, int h, const Geo& geo, const AtrousTaps& taps, const uint2* __restrict__ color, const uint32_t* __restrict__ var_tex, uint2* __restrict__ out_color, uint32_t* __restrict__ out_var, uint32_t* __restrict__ out_diff, uint32_t* __restrict__ out_spec, int step) {
   size_t i = (size_t)y * w + x;
   uint2 cc = color[i];
   f3 diff_c = col_diff(cc), spec_c = col_spec(cc);
@@ -487,7 +484,223 @@ struct DnAtrousF {
   if (out_diff) out_diff[i] = pd;
   if (out_spec) out_spec[i] = ps;
 }
+
+template <class Geo>
+struct DnAtrousF {
+  static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, AtrousTaps taps, const uint2* __restrict__ color, const uint32_t* __restrict__ var_tex, uint2* __restrict__ out_color, uint32_t* __restrict__ out_var, uint32_t* __restrict__ out_diff, uint32_t* __restrict__ out_spec, int step) {
+  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
+  if (!inb(x, y, w, h)) return;
+  atrous_px(x, y, w, h, geo, taps, color, var_tex, out_color, out_var, out_diff, out_spec, step);
+}
 };
+
+// The a-trous iteration over tiles staged in shared memory, for steps up to
+// kAtrousTileMaxStep. The per-pixel form above decodes every tap anew: two R11G11B10
+// words, two luminances, and from the raw G-buffer an octahedral normal, 16 times per
+// pixel (235 warp instructions per tap, and a third of the stalls instruction fetch).
+// Here a block decodes each pixel of its tile and halo once. The tile is 64
+// consecutive columns of 8 rows that lie `step` apart, so that at every step the halo
+// is four rows and 4 * step columns, loads stay coalesced and 1.6 (step 1) to 3 (step
+// 16) pixels are decoded per output pixel.
+//
+// A staged pixel is 48 bytes, diffuse and specular channel interleaved (a stride of 12
+// words: the eight lanes of each phase of a 128-bit load fall on distinct banks), plus
+// the two variances. The interleaving gives both channels' arithmetic as register
+// pairs, and the paired binary32 instructions (one IEEE operation per component, the
+// same bits) halve the issue slots of the parts that run per channel.
+//
+// Two things the per-pixel form guards per tap are settled per block. A block is
+// `tame` when every staged colour and variance is finite, no variance is negative,
+// every depth is 0 or of a magnitude in [2^-70, 2^70] and no fwidth_z of the tile is
+// negative or not finite. Then no weight exponent is positive or NaN, and quotients
+// may be formed with a shared reciprocal (div_shared). Other blocks run the per-pixel
+// form.
+//
+// Bound by binary32 arithmetic: 1,834 warp instructions per 32 pixels (3,770 in the
+// per-pixel form) at 60 % issue, FMA pipe 49 % (the paired instructions take two of its
+// cycles). 1920x1080 from the raw G-buffer: 337 -> 133 us per iteration; from the surface
+// planes at 1280x720: 124 -> 65 us. Measured and not kept: a loop over the four tap rows
+// instead of unrolled taps (416 us for three iterations against 398), 3 or 2 blocks per SM
+// (423, 534), 16 rows by 512 threads (416), 4 rows by 128 (446), staging unrolled by two
+// (408). Above kAtrousTileMaxStep the halo outgrows the tile and the per-pixel form
+// runs; recorded (batched) jobs, whose tile shape the batch chooses, run it too.
+constexpr int kAtrousTileMaxStep = 16;
+constexpr int kAtrousTileX = 64, kAtrousTileRows = 8;
+
+struct AtrousPx {
+  float4 a;  // diffuse.r, specular.r, diffuse.g, specular.g
+  float4 b;  // diffuse.b, specular.b, diffuse and specular luminance
+  float4 c;  // normal, depth
+};
+
+__device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
+// a * b + c per component with the product rounded before the sum. The compiler fuses a
+// paired multiply and a paired add (also the explicitly rounded intrinsics, and a
+// fused multiply-add by a literal 1) into one fused multiply-add, which rounds once.
+// A factor of 1 that only the host knows, a kernel argument, keeps the two apart.
+__device__ __forceinline__ float2 madd2(float2 a, float2 b, float2 c, float one) {
+  return __ffma2_rn(__fmul2_rn(a, b), bc2(one), c);
+}
+
+// a / b, correctly rounded, from r = RN(1 / b): q = RN(a r), then one correction by the
+// exact remainder (Markstein 1990). An exhaustive comparison over all 2^46 pairs of
+// binary32 mantissas found no difference from the IEEE quotient; the remainder must
+// not underflow, so a is 0 or of magnitude at least 2^-100 while b is of ordinary size
+// (|b| in [2^-30, 2^40] here), or the quotient of a smaller a may be off by an ulp.
+__device__ __forceinline__ float div_shared(float a, float b, float r) {
+  const float q = a * r;
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
+struct AtrousOut {
+  uint2* __restrict__ color;
+  uint32_t* __restrict__ var;
+  uint32_t* __restrict__ diff;
+  uint32_t* __restrict__ spec;
+};
+
+// One output pixel of a tame block; s is the staged tile, li the pixel's place in it,
+// pw the tile's row pitch. CHECK: the footprint may leave the image.
+template <bool CHECK>
+__device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* sv, int li, int pw, int x, int y,
+                                               int w, int h, float fwz, float3 td, int step, const AtrousOut& o, float one) {
+  const float4 ca = s[li].a, cb = s[li].b, cc = s[li].c;
+  const float2 cv = sv[li];
+  const float eps = 1e-8f;
+  const float2 neg_lum = make_float2(-cb.z, -cb.w);
+  const float2 rcp_l = make_float2(1.0f / (4.0f * sqrt_(cv.x) + eps), 1.0f / (4.0f * sqrt_(cv.y) + eps));
+  const float den[3] = {fwz * td.x + eps, fwz * td.y + eps, fwz * td.z + eps};
+  const float rden[3] = {1.0f / den[0], 1.0f / den[1], 1.0f / den[2]};
+  float2 r = make_float2(ca.x, ca.y), g = make_float2(ca.z, ca.w), b = make_float2(cb.x, cb.y), v = cv,
+         ws = bc2(1.0f);
+  const float kw[3] = {1.0f, 2.0f / 3.0f, 1.0f / 6.0f};
+  const float M = 12582912.0f;  // 1.5 * 2^23: the shifter of exp2_select
+#pragma unroll
+  for (int oy = -2; oy <= 2; ++oy) {
+    if (oy == 0) continue;
+    if (CHECK && !inb(0, y + oy * step, 1, h)) continue;
+#pragma unroll
+    for (int ox = -2; ox <= 2; ++ox) {
+      if (ox == 0) continue;
+      if (CHECK && !inb(x + ox * step, 0, w, 1)) continue;
+      const int ax = ox < 0 ? -ox : ox, ay = oy < 0 ? -oy : oy, cls = ax + ay - 2;
+      const int j = li + oy * pw + ox * step;
+      const float4 ta = s[j].a, tb = s[j].b, tc = s[j].c;
+      const float2 tv = sv[j];
+      const float q = div_shared(fabsf(tc.w - cc.w), den[cls], rden[cls]);
+      const float2 nxy = __fmul2_rn(make_float2(cc.x, cc.y), make_float2(tc.x, tc.y));
+      float wn = __saturatef(nxy.x + nxy.y + cc.z * tc.z);
+      wn = pow_2k(wn, 7);
+      // exponent -(|dl| rcp_l + q): every term is finite and non-negative
+      const float2 dl = __fmul2_rn(__fadd2_rn(make_float2(tb.z, tb.w), neg_lum), rcp_l);
+      float2 e = __ffma2_rn(make_float2(fabsf(dl.x), fabsf(dl.y)), bc2(one), bc2(q));
+      e = __fmul2_rn(e, bc2(-VLT_LOG2E));
+      // exp2_select<false> for arguments <= 0: below -151 the clamp itself gives 0
+      e = make_float2(fmax_(e.x, -151.0f), fmax_(e.y, -151.0f));
+      const float2 t = __fadd2_rn(e, bc2(M));
+      const float2 f = __fadd2_rn(e, __ffma2_rn(t, bc2(-1.0f), bc2(M)));
+      float2 p = madd2(bc2(VLT_EXP2_C6), f, bc2(VLT_EXP2_C5), one);
+      p = madd2(p, f, bc2(VLT_EXP2_C4), one);
+      p = madd2(p, f, bc2(VLT_EXP2_C3), one);
+      p = madd2(p, f, bc2(VLT_EXP2_C2), one);
+      p = madd2(p, f, bc2(VLT_EXP2_C1), one);
+      p = madd2(p, f, bc2(VLT_EXP2_C0), one);
+      // 2^n as 2^e1 2^e2, e1 = max(n, -126): the integers sit in the shifted sums' low bits
+      const int tx = (int)as_uint(t.x), ty = (int)as_uint(t.y);
+      const int lo = 0x4B400000 - 126;
+      const int ex = tx < lo ? lo : tx, ey = ty < lo ? lo : ty;
+      const float2 s1 = make_float2(as_float(((uint32_t)ex << 23) + 0x3F800000u),
+                                    as_float(((uint32_t)ey << 23) + 0x3F800000u));
+      const float2 s2 = make_float2(as_float(((uint32_t)(tx - ex) << 23) + 0x3F800000u),
+                                    as_float(((uint32_t)(ty - ey) << 23) + 0x3F800000u));
+      p = __fmul2_rn(__fmul2_rn(p, s1), s2);
+      const float2 wt = __fmul2_rn(bc2(kw[ay] * kw[ax]), __fmul2_rn(bc2(wn), p));
+      r = madd2(wt, make_float2(ta.x, ta.y), r, one);
+      g = madd2(wt, make_float2(ta.z, ta.w), g, one);
+      b = madd2(wt, make_float2(tb.x, tb.y), b, one);
+      v = madd2(__fmul2_rn(wt, wt), tv, v, one);
+      ws = __ffma2_rn(wt, bc2(one), ws);
+    }
+  }
+  // 1 <= ws <= 17; a sum too small for div_shared is stored as 0 either way
+  const float2 rw = make_float2(1.0f / ws.x, 1.0f / ws.y), w2 = __fmul2_rn(ws, ws);
+  const uint32_t pd = pack_r11g11b10(
+      mk3(div_shared(r.x, ws.x, rw.x), div_shared(g.x, ws.x, rw.x), div_shared(b.x, ws.x, rw.x)));
+  const uint32_t ps = pack_r11g11b10(
+      mk3(div_shared(r.y, ws.y, rw.y), div_shared(g.y, ws.y, rw.y), div_shared(b.y, ws.y, rw.y)));
+  const size_t i = (size_t)y * w + x;
+  if (o.color) o.color[i] = make_uint2(pd, ps);
+  if (o.var) o.var[i] = pack_half2(mk2(v.x / w2.x, v.y / w2.y));
+  if (o.diff) o.diff[i] = pd;
+  if (o.spec) o.spec[i] = ps;
+}
+
+// Bytes of a block's staged tile at a step.
+static inline size_t atrous_tile_bytes(int step) {
+  return (size_t)(kAtrousTileX + 4 * step) * (kAtrousTileRows + 4) * (sizeof(AtrousPx) + sizeof(float2));
+}
+
+template <class Geo, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
+    k_atrous_tile(int w, int h, Geo geo, AtrousTaps taps, const uint2* __restrict__ color,
+                  const uint32_t* __restrict__ var_tex, AtrousOut o, int step, uint32_t pitch_inv, float one) {
+  extern __shared__ float4 smem[];
+  const int pw = kAtrousTileX + 4 * step, np = pw * (kAtrousTileRows + 4);
+  AtrousPx* s = reinterpret_cast<AtrousPx*>(smem);
+  float2* sv = reinterpret_cast<float2*>(s + np);
+  const int tid = (int)threadIdx.x;
+  // Tile rows: blockIdx.y counts (group of 8 * step image rows, phase within it).
+  const int group = (int)blockIdx.y / step, phase = (int)blockIdx.y - group * step;
+  const int x0 = (int)blockIdx.x * kAtrousTileX, y0 = group * (kAtrousTileRows * step) + phase;
+  bool tame = true;
+  for (int k = tid; k < np; k += NT) {
+    const int row = (int)__umulhi((uint32_t)k, pitch_inv), col = k - row * pw;  // k / pw (host: exact for k < np)
+    const int gx = x0 + col - 2 * step, gy = y0 + (row - 2) * step;
+    if (!inb(gx, gy, w, h)) continue;  // never read: the border form checks every tap
+    const size_t i = (size_t)gy * w + gx;
+    const uint2 cw = color[i];
+    const uint32_t vw = var_tex[i];
+    const f3 n = geo.normal(i);
+    const float dep = geo.dep(i);
+    const f3 d = col_diff(cw), sp = col_spec(cw);
+    AtrousPx px;
+    px.a = make_float4(d.x, sp.x, d.y, sp.y);
+    px.b = make_float4(d.z, sp.z, luminance(d), luminance(sp));
+    px.c = make_float4(n.x, n.y, n.z, dep);
+    s[k] = px;
+    const f2 v = unpack_half2(vw);
+    sv[k] = make_float2(v.x, v.y);
+    const float ad = fabsf(dep);
+    // exponent code 31: an infinity or a NaN
+    const bool special = (cw.x & 0x7C0u) == 0x7C0u || (cw.x & 0x3E0000u) == 0x3E0000u ||
+                         (cw.x & 0xF8000000u) == 0xF8000000u || (cw.y & 0x7C0u) == 0x7C0u ||
+                         (cw.y & 0x3E0000u) == 0x3E0000u || (cw.y & 0xF8000000u) == 0xF8000000u;
+    tame = tame && !special && v.x >= 0.0f && v.y >= 0.0f && v.x < 1e6f && v.y < 1e6f &&
+           (dep == 0.0f || (ad >= 0x1p-70f && ad <= 0x1p70f));
+    if (row >= 2 && row < kAtrousTileRows + 2 && col >= 2 * step && col < kAtrousTileX + 2 * step) {
+      const float fz = geo.fwz(i);
+      tame = tame && fz >= 0.0f && fz < 1e6f;
+    }
+  }
+  tame = __syncthreads_and(tame);
+  const float3 td = make_float3(taps.dist[5], taps.dist[4], taps.dist[0]);
+  const bool interior = x0 - 2 * step >= 0 && x0 + kAtrousTileX - 1 + 2 * step <= w - 1 && y0 - 2 * step >= 0 &&
+                        y0 + (kAtrousTileRows + 1) * step <= h - 1;
+  const int tx = tid & (kAtrousTileX - 1), ty = tid / kAtrousTileX;
+#pragma unroll 1
+  for (int row = ty; row < kAtrousTileRows; row += NT / kAtrousTileX) {
+    const int x = x0 + tx, y = y0 + row * step;
+    if (!inb(x, y, w, h)) return;
+    if (!tame) {
+      atrous_px(x, y, w, h, geo, taps, color, var_tex, o.color, o.var, o.diff, o.spec, step);
+      continue;
+    }
+    const float fwz = geo.fwz((size_t)y * w + x);
+    const int li = (row + 2) * pw + tx + 2 * step;
+    if (interior) atrous_tile_px<false>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
+    else atrous_tile_px<true>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
+  }
+}
 
 struct SplitColorF {
   static __device__ __forceinline__ void run(int x0, int y0, int n, const uint2* __restrict__ color, uint32_t* __restrict__ d, uint32_t* __restrict__ s) {
@@ -555,6 +768,31 @@ void launch_dn_fallback(const Exec& ex, int w, int h, const GeoArgs& ga, const u
                                   (uint2*)out_color, out_var);
 }
 
+template <class Geo>
+static void launch_atrous_tile(const Exec& ex, int w, int h, const Geo& geo, const AtrousTaps& taps,
+                               const uint32_t* color, const uint32_t* var, uint32_t* out_color, uint32_t* out_var,
+                               uint32_t* out_diff, uint32_t* out_spec, int step) {
+  if (w <= 0 || h <= 0) return;
+  if (ex.launches) ++*ex.launches;
+  const int pw = kAtrousTileX + 4 * step;
+  const unsigned groups = (unsigned)((h + kAtrousTileRows * step - 1) / (kAtrousTileRows * step));
+  const dim3 grid((unsigned)((w + kAtrousTileX - 1) / kAtrousTileX), groups * (unsigned)step, 1);
+  // ceil(2^32 / pw): the high word of k * pitch_inv is k / pw for k below 2^16
+  const uint32_t pitch_inv = (uint32_t)(((uint64_t)1 << 32) / (uint32_t)pw + 1u);
+  const AtrousOut o = {(uint2*)out_color, out_var, out_diff, out_spec};
+  const size_t bytes = atrous_tile_bytes(step);
+  auto run = [&](auto kernel, int threads) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)atrous_tile_bytes(kAtrousTileMaxStep));
+    kernel<<<grid, threads, bytes, ex.stream>>>(w, h, geo, taps, (const uint2*)color, var, o, step, pitch_inv, 1.0f);
+  };
+  // One output row per thread while there are few tiles per SM (a block's own latency is
+  // then the pass), two rows on fewer threads for more. Five iterations, 256 / 512
+  // threads: 320x180 73 / 54 us, 640x360 134 / 114 us, 854x480 193 / 175 us; three at
+  // 1920x1080 398 / 428 us.
+  if ((int)(grid.x * grid.y) <= 8 * device_sm_count()) run(k_atrous_tile<Geo, 512>, 512);
+  else run(k_atrous_tile<Geo, 256>, 256);
+}
+
 void launch_dn_atrous(const Exec& ex, int w, int h, const GeoArgs& ga, const uint32_t* color, const uint32_t* var,
                       uint32_t* out_color, uint32_t* out_var, uint32_t* out_diff, uint32_t* out_spec, int step) {
   AtrousTaps taps;
@@ -566,6 +804,13 @@ void launch_dn_atrous(const Exec& ex, int w, int h, const GeoArgs& ga, const uin
       float fx = (float)(ox * step), fy = (float)(oy * step);
       taps.dist[k++] = sqrtf(fx * fx + fy * fy);  // correctly rounded, == device sqrt.rn
     }
+  }
+  if (!ex.rec && step <= kAtrousTileMaxStep) {
+    if (ga.nd)
+      launch_atrous_tile(ex, w, h, surf_geo(ga, w, h), taps, color, var, out_color, out_var, out_diff, out_spec, step);
+    else
+      launch_atrous_tile(ex, w, h, raw_geo(ga, w, h), taps, color, var, out_color, out_var, out_diff, out_spec, step);
+    return;
   }
   if (ga.nd)
     launch2d<DnAtrousF<GeoSurface>>(ex, "dn_atrous", w, h, w, h, surf_geo(ga, w, h), taps, (const uint2*)color, var,
