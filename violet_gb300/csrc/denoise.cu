@@ -4,6 +4,7 @@
 // Colour history is a packed uint2 {diffuse, specular} of R11G11B10 words (one
 // 64-bit access per tap), moments/variance are half2, history length is R8_UNORM.
 // Kernels are templated on the geometry source (GeoRaw / GeoSurface).
+#include "short_history.cuh"
 #include "vlt_internal.h"
 
 namespace vlt {
@@ -19,14 +20,12 @@ struct EdgeStop {
   f3 normal_center;
   f2 lumi_center;
   f2 lumi_rcp;
-  bool use_lumi;
   float sigma_z;
   int sigma_n_log2;  // sigma_n = 2^k (128 -> 7, 32 -> 5)
 
   __device__ __forceinline__ void set_lumi(f2 lumi, f2 var) {
     const float sigma_l = 4.0f;
     const float eps = 1e-8f;
-    use_lumi = true;
     lumi_center = lumi;
     f2 sd = mk2(sqrt_(var.x), sqrt_(var.y));
     lumi_rcp = mk2(1.0f / (sigma_l * sd.x + eps), 1.0f / (sigma_l * sd.y + eps));
@@ -38,11 +37,8 @@ struct EdgeStop {
     float wz = -dist_z / ((sigma_z * fwidth_z) * tap_dist + eps);
     float n_dot = saturate(dot3(normal_center, normal));
     float wn = pow_2k(n_dot, sigma_n_log2);
-    f2 wl = mk2(0.0f, 0.0f);
-    if (use_lumi) {
-      f2 dl = mk2(fabs_(lumi.x - lumi_center.x), fabs_(lumi.y - lumi_center.y));
-      wl = mk2(-dl.x * lumi_rcp.x, -dl.y * lumi_rcp.y);
-    }
+    f2 dl = mk2(fabs_(lumi.x - lumi_center.x), fabs_(lumi.y - lumi_center.y));
+    f2 wl = mk2(-dl.x * lumi_rcp.x, -dl.y * lumi_rcp.y);
     return mk2(wn * exp_(wl.x + wz), wn * exp_(wl.y + wz));
   }
 };
@@ -54,7 +50,6 @@ __device__ __forceinline__ EdgeStop make_edge_stop(float depth, float fwidth_z, 
   e.normal_center = normal;
   e.lumi_center = mk2(0.0f, 0.0f);
   e.lumi_rcp = mk2(0.0f, 0.0f);
-  e.use_lumi = false;
   e.sigma_z = 1.0f;
   e.sigma_n_log2 = 7;
   return e;
@@ -272,53 +267,63 @@ __device__ __forceinline__ float quad_max_len(const uint8_t* __restrict__ len, i
 
 // --------------------------------------------------------- disocclusion fix
 
+// Sums of the short-history filters (the weight without luminance terms is the same for
+// both channels), and that weight.
+struct FilterSums {
+  float w = 0.0f;
+  f3 d = mk3(0.0f), s = mk3(0.0f);
+  f2 m = mk2(0.0f, 0.0f);
+  __device__ __forceinline__ void add(float wt, uint2 c, uint32_t mom) {
+    w = w + wt;
+    d = d + col_diff(c) * wt;
+    s = s + col_spec(c) * wt;
+    m = m + unpack_half2(mom) * wt;
+  }
+};
+template <class Geo>
+__device__ __forceinline__ float short_weight(const ShortPixel& c, const Geo& geo, size_t j, float tap_dist,
+                                              int sigma_n_log2) {
+  const float wz = -fabs_(geo.dep(j) - c.depth) / (c.fz_sigma * tap_dist + 1e-8f);
+  return pow_2k(saturate(dot3(c.normal, geo.normal(j))), sigma_n_log2) * exp_(wz);
+}
+
 // relax_disocclusion_fix.hlsl:27-122. Pixels without geometry (history 0) are not
 // written by the shader; here they get zeros.
 template <class Geo>
 struct DnFixF {
+  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const uint8_t* __restrict__ len_tex, const uint2* __restrict__ color, const uint32_t* __restrict__ mom, uint2* __restrict__ out_color, uint32_t* __restrict__ out_mom) {
-  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
-  if (!inb(x, y, w, h)) return;
-  size_t i = (size_t)y * w + x;
-  float hl = unorm8_load(len_tex[i]);
-  float qmax = quad_max_len(len_tex, x, y, w, h);
-  if (hl == 0.0f) {
-    out_color[i] = make_uint2(0u, 0u);
-    out_mom[i] = 0u;
-    return;
+  __shared__ ShortStage<2> st;
+  const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
+  const bool inside = inb(x, y, w, h);
+  const size_t i = inside ? (size_t)y * w + x : 0;
+  const float hl = inside ? unorm8_load(len_tex[i]) : 0.0f;
+  const float qmax = inside ? quad_max_len(len_tex, x, y, w, h) : 0.0f;
+  const bool is_short = hl != 0.0f && qmax < 4.0f * VLT_HISTORY_LEN_UNIT;
+  ShortPixel c = {mk3(0.0f), 0.0f, 0.0f, x, y, 0};
+  if (is_short) {
+    c.stride = f2i_rz((14.0f * VLT_HISTORY_LEN_UNIT) / qmax);
+    c.depth = geo.dep(i);
+    c.fz_sigma = 5.0f * geo.fwz(i);
+    c.normal = geo.normal(i);
+  } else if (inside) {
+    out_color[i] = hl == 0.0f ? make_uint2(0u, 0u) : color[i];
+    out_mom[i] = hl == 0.0f ? 0u : mom[i];
   }
-  hl = qmax;
-  if (hl < 4.0f * VLT_HISTORY_LEN_UNIT) {
-    EdgeStop es = make_edge_stop(geo.dep(i), geo.fwz(i), geo.normal(i));
-    es.sigma_z = 5.0f;
-    es.sigma_n_log2 = 5;
-    f2 ws = mk2(0.0f, 0.0f);
-    f3 dsum = mk3(0.0f), ssum = mk3(0.0f);
-    f2 msum = mk2(0.0f, 0.0f);
-    const int stride = f2i_rz((14.0f * VLT_HISTORY_LEN_UNIT) / hl);
-    for (int oy = -2; oy <= 2; ++oy) {
-      for (int ox = -2; ox <= 2; ++ox) {
-        int offx = ox * stride, offy = oy * stride;
-        int cx = x + offx, cy = y + offy;
-        if (!(cx >= 0 && cy >= 0 && cx <= w - 1 && cy <= h - 1)) continue;
-        size_t j = (size_t)cy * w + cx;
-        f2 wt = es.weight(length2(mk2((float)offx, (float)offy)), geo.dep(j), geo.normal(j), mk2(0.0f, 0.0f));
-        uint2 c = color[j];
-        f2 m = unpack_half2(mom[j]);
-        ws = ws + wt;
-        dsum = dsum + col_diff(c) * wt.x;
-        ssum = ssum + col_spec(c) * wt.y;
-        msum = msum + m * wt;
-      }
-    }
-    f3 dd = dsum / ws.x;
-    f3 sd = ssum / ws.y;
-    f2 md = msum / ws;
-    out_color[i] = make_uint2(pack_r11g11b10(dd), pack_r11g11b10(sd));
-    out_mom[i] = pack_half2(md);
-  } else {
-    out_color[i] = color[i];
-    out_mom[i] = mom[i];
+  FilterSums t;
+  filter_short_pixels<2>(
+      is_short, c, w, h, st,
+      [&](const ShortPixel& cc, size_t j, int ox, int oy) {
+        return short_weight(cc, geo, j, length2(mk2((float)(ox * cc.stride), (float)(oy * cc.stride))), 5);
+      },
+      [&](float wt, size_t j, bool ok) {
+        const uint2 cj = color[j];
+        const uint32_t mj = mom[j];
+        if (ok) t.add(wt, cj, mj);
+      });
+  if (is_short) {
+    out_color[i] = make_uint2(pack_r11g11b10(t.d / t.w), pack_r11g11b10(t.s / t.w));
+    out_mom[i] = pack_half2(mk2(t.m.x / t.w, t.m.y / t.w));
   }
 }
 };
@@ -375,54 +380,50 @@ struct DnFastClampF {
 // svgf_spatial_fallback_filter.hlsl:25-125. History-0 pixels get zeros.
 template <class Geo>
 struct DnFallbackF {
+  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const uint8_t* __restrict__ len_tex, const uint2* __restrict__ color, const uint32_t* __restrict__ mom, uint2* __restrict__ out_color, uint32_t* __restrict__ out_var) {
-  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
-  if (!inb(x, y, w, h)) return;
-  size_t i = (size_t)y * w + x;
-  float hl = unorm8_load(len_tex[i]);
-  float qmax = quad_max_len(len_tex, x, y, w, h);
-  if (hl == 0.0f) {
-    out_color[i] = make_uint2(0u, 0u);
-    out_var[i] = 0u;
-    return;
+  __shared__ ShortStage<3> st;
+  const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
+  const bool inside = inb(x, y, w, h);
+  const size_t i = inside ? (size_t)y * w + x : 0;
+  const float own = inside ? unorm8_load(len_tex[i]) : 0.0f;
+  const float hl = inside ? quad_max_len(len_tex, x, y, w, h) : 0.0f;
+  const bool is_short = own != 0.0f && hl < 4.0f * VLT_HISTORY_LEN_UNIT;
+  ShortPixel c = {mk3(0.0f), 0.0f, 0.0f, x, y, 1};
+  if (is_short) {
+    c.depth = geo.dep(i);
+    c.fz_sigma = 1.0f * (geo.fwz(i) * 3.0f);
+    c.normal = geo.normal(i);
   }
-  hl = qmax;
-  f3 dd, sd;
-  f2 md;
-  if (hl < 4.0f * VLT_HISTORY_LEN_UNIT) {
-    EdgeStop es = make_edge_stop(geo.dep(i), geo.fwz(i) * 3.0f, geo.normal(i));
-    f2 ws = mk2(0.0f, 0.0f);
-    f3 dsum = mk3(0.0f), ssum = mk3(0.0f);
-    f2 msum = mk2(0.0f, 0.0f);
-    for (int oy = -3; oy <= 3; ++oy) {
-      for (int ox = -3; ox <= 3; ++ox) {
-        int cx = x + ox, cy = y + oy;
-        if (!(cx >= 0 && cy >= 0 && cx <= w - 1 && cy <= h - 1)) continue;
-        size_t j = (size_t)cy * w + cx;
-        float wt = es.weight(length2(mk2((float)ox, (float)oy)), geo.dep(j), geo.normal(j), mk2(0.0f, 0.0f)).x;
-        uint2 c = color[j];
-        f2 m = unpack_half2(mom[j]);
-        ws = mk2(ws.x + wt, ws.y + wt);
-        dsum = dsum + col_diff(c) * wt;
-        ssum = ssum + col_spec(c) * wt;
-        msum = msum + m * wt;
-      }
+  const auto finish = [&](f3 dd, f3 sd, f2 md) {
+    f2 fst = mk2(luminance(dd), luminance(sd));
+    f2 var = mk2(fmax_(md.x - fst.x * fst.x, 0.0f), fmax_(md.y - fst.y * fst.y, 0.0f));
+    float boost = fmax_(1.0f, (4.0f * VLT_HISTORY_LEN_UNIT) / hl);
+    var = var * boost;
+    out_color[i] = make_uint2(pack_r11g11b10(dd), pack_r11g11b10(sd));
+    out_var[i] = pack_half2(var);
+  };
+  if (inside && !is_short) {
+    if (own == 0.0f) {
+      out_color[i] = make_uint2(0u, 0u);
+      out_var[i] = 0u;
+    } else {
+      const uint2 cc = color[i];
+      finish(col_diff(cc), col_spec(cc), unpack_half2(mom[i]));
     }
-    dd = dsum / ws.x;
-    sd = ssum / ws.y;
-    md = msum / ws;
-  } else {
-    uint2 c = color[i];
-    dd = col_diff(c);
-    sd = col_spec(c);
-    md = unpack_half2(mom[i]);
   }
-  f2 fst = mk2(luminance(dd), luminance(sd));
-  f2 var = mk2(fmax_(md.x - fst.x * fst.x, 0.0f), fmax_(md.y - fst.y * fst.y, 0.0f));
-  float boost = fmax_(1.0f, (4.0f * VLT_HISTORY_LEN_UNIT) / hl);
-  var = var * boost;
-  out_color[i] = make_uint2(pack_r11g11b10(dd), pack_r11g11b10(sd));
-  out_var[i] = pack_half2(var);
+  FilterSums t;
+  filter_short_pixels<3>(
+      is_short, c, w, h, st,
+      [&](const ShortPixel& cc, size_t j, int ox, int oy) {
+        return short_weight(cc, geo, j, length2(mk2((float)ox, (float)oy)), 7);
+      },
+      [&](float wt, size_t j, bool ok) {
+        const uint2 cj = color[j];
+        const uint32_t mj = mom[j];
+        if (ok) t.add(wt, cj, mj);
+      });
+  if (is_short) finish(t.d / t.w, t.s / t.w, mk2(t.m.x / t.w, t.m.y / t.w));
 }
 };
 

@@ -18,6 +18,7 @@
 // divides by the square root of a variance computed as E[l^2] - E[l]^2, which
 // cancels near zero, so a last-bit difference upstream can change a weight
 // completely.
+#include "short_history.cuh"
 #include "vlt_internal.h"
 
 namespace vlt {
@@ -148,21 +149,8 @@ struct EdgeStopFast {
   float depth_center, fz_sigma;  // sigma_z * fwidth_z
   f3 normal_center;
   f2 lumi_center, lumi_rcp;
-  bool use_lumi;
   int sigma_n_log2;
 
-  __device__ __forceinline__ f2 weight(float tap_dist, float depth, f3 normal, f2 lumi) const {
-    float dist_z = fabsf(depth - depth_center);
-    float wz = -dist_z / fma_(fz_sigma, tap_dist, 1e-8f);
-    float n_dot = saturate(fma_(normal_center.z, normal.z, fma_(normal_center.y, normal.y, normal_center.x * normal.x)));
-    float wn = pow_2k(n_dot, sigma_n_log2);
-    float ax = wz, ay = wz;
-    if (use_lumi) {
-      ax = fma_(-fabsf(lumi.x - lumi_center.x), lumi_rcp.x, wz);
-      ay = fma_(-fabsf(lumi.y - lumi_center.y), lumi_rcp.y, wz);
-    }
-    return mk2(wn * exp_fma(ax), wn * exp_fma(ay));
-  }
   // The a-trous weight, in base 2 and with the kernel weight k: the depth term as
   // -dist_z * r_z with r_z = log2(e) / (fz_sigma * d + 1e-8) precomputed by the caller
   // for the tap's distance d (the a-trous taps have only three distinct distances),
@@ -184,7 +172,6 @@ __device__ __forceinline__ EdgeStopFast make_es(float depth, float fwidth_z, flo
   e.normal_center = normal;
   e.lumi_center = mk2(0.0f, 0.0f);
   e.lumi_rcp = mk2(0.0f, 0.0f);
-  e.use_lumi = false;
   e.sigma_n_log2 = n_log2;
   return e;
 }
@@ -443,60 +430,80 @@ struct Dn32TemporalF {
 
 // ----------------------------------------------------------- disocclusion fix
 
+// Sums of the short-history filters (the weight without luminance terms is the same for
+// both channels), and that weight.
+template <bool CENTERED>
+struct FilterSums {
+  float w = 0.0f;
+  f3 d = mk3(0.0f), s = mk3(0.0f);
+  f2 m = mk2(0.0f, 0.0f);
+  __device__ __forceinline__ void add(float wt, const Rec& r, f2 kshift) {
+    w = w + wt;
+    d = fma3(wt, r.d, d);
+    s = fma3(wt, r.s, s);
+    if (CENTERED) {
+      const f2 e = lum2(r.d, r.s) - kshift;
+      m = mk2(fma_(wt, fma_(e.x, e.x, r.aux.x), m.x), fma_(wt, fma_(e.y, e.y, r.aux.y), m.y));
+    } else {
+      m = mk2(fma_(wt, r.aux.x, m.x), fma_(wt, r.aux.y, m.y));
+    }
+  }
+};
+template <class Geo>
+__device__ __forceinline__ float short_weight(const ShortPixel& c, const Geo& geo, size_t j, float tap_dist,
+                                              int sigma_n_log2) {
+  const float wz = -fabsf(geo.dep(j) - c.depth) / fma_(c.fz_sigma, tap_dist, 1e-8f);
+  const f3 n = geo.normal(j);
+  const float n_dot = saturate(fma_(c.normal.z, n.z, fma_(c.normal.y, n.y, c.normal.x * n.x)));
+  return pow_2k(n_dot, sigma_n_log2) * exp_fma(wz);
+}
+
 template <class Geo, int FORM>
 struct Dn32FixF {
+  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
   using R = typename DnT<FORM>::R;
   using N = typename DnT<FORM>::N;
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const N* __restrict__ len, const R* __restrict__ in, R* __restrict__ out) {
-  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
-  if (!inb(x, y, w, h)) return;
-  size_t i = (size_t)y * w + x;
-  float hl = ld_len(len, i);
-  float qmax = quad_max_len(len, x, y, w, h);
-  if (hl == 0.0f) {
-    store_rec(out, i, mk3(0.0f), mk3(0.0f), mk2(0.0f, 0.0f));
-    return;
-  }
-  hl = qmax;
-  if (hl < 4.0f * VLT_HISTORY_LEN_UNIT) {
-    EdgeStopFast es = make_es(geo.dep(i), geo.fwz(i), 5.0f, geo.normal(i), 5);
-    f2 ws = mk2(0.0f, 0.0f);
-    f3 dsum = mk3(0.0f), ssum = mk3(0.0f);
-    f2 msum = mk2(0.0f, 0.0f);
-    f2 kshift = mk2(0.0f, 0.0f);  // centered form: the centre record's luminance
+  __shared__ ShortStage<2> st;
+  const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
+  const bool inside = inb(x, y, w, h);
+  const size_t i = inside ? (size_t)y * w + x : 0;
+  const float hl = inside ? ld_len(len, i) : 0.0f;
+  const float qmax = inside ? quad_max_len(len, x, y, w, h) : 0.0f;
+  const bool is_short = hl != 0.0f && qmax < 4.0f * VLT_HISTORY_LEN_UNIT;
+  ShortPixel c = {mk3(0.0f), 0.0f, 0.0f, x, y, 0};
+  FilterSums<Centered<FORM>::value> t;
+  f2 kshift = mk2(0.0f, 0.0f);  // centered form: the centre record's luminance
+  if (is_short) {
+    c.stride = f2i_rz((14.0f * VLT_HISTORY_LEN_UNIT) / qmax);
+    c.depth = geo.dep(i);
+    c.fz_sigma = 5.0f * geo.fwz(i);
+    c.normal = geo.normal(i);
     if (Centered<FORM>::value) {
       const Rec rc = load_rec(in, i);
       kshift = lum2(rc.d, rc.s);
     }
-    const int stride = f2i_rz((14.0f * VLT_HISTORY_LEN_UNIT) / hl);
-    for (int oy = -2; oy <= 2; ++oy) {
-      for (int ox = -2; ox <= 2; ++ox) {
-        int offx = ox * stride, offy = oy * stride;
-        int cx = x + offx, cy = y + offy;
-        if (!(cx >= 0 && cy >= 0 && cx <= w - 1 && cy <= h - 1)) continue;
-        size_t j = (size_t)cy * w + cx;
-        f2 wt = es.weight(length2(mk2((float)offx, (float)offy)), geo.dep(j), geo.normal(j), mk2(0.0f, 0.0f));
-        Rec r = load_rec(in, j);
-        ws = ws + wt;
-        dsum = fma3(wt.x, r.d, dsum);
-        ssum = fma3(wt.y, r.s, ssum);
-        if (Centered<FORM>::value) {
-          const f2 e = lum2(r.d, r.s) - kshift;
-          msum = mk2(fma_(wt.x, fma_(e.x, e.x, r.aux.x), msum.x), fma_(wt.y, fma_(e.y, e.y, r.aux.y), msum.y));
-        } else {
-          msum = mk2(fma_(wt.x, r.aux.x, msum.x), fma_(wt.y, r.aux.y, msum.y));
-        }
-      }
-    }
-    const f3 dfix = dsum * (1.0f / ws.x), sfix = ssum * (1.0f / ws.y);
-    f2 mfix = mk2(msum.x / ws.x, msum.y / ws.y);
+  } else if (inside) {
+    if (hl == 0.0f) store_rec(out, i, mk3(0.0f), mk3(0.0f), mk2(0.0f, 0.0f));
+    else copy_rec(out, in, i);
+  }
+  filter_short_pixels<2>(
+      is_short, c, w, h, st,
+      [&](const ShortPixel& cc, size_t j, int ox, int oy) {
+        return short_weight(cc, geo, j, length2(mk2((float)(ox * cc.stride), (float)(oy * cc.stride))), 5);
+      },
+      [&](float wt, size_t j, bool ok) {
+        const Rec r = load_rec(in, j);
+        if (ok) t.add(wt, r, kshift);
+      });
+  if (is_short) {
+    const f3 dfix = t.d * (1.0f / t.w), sfix = t.s * (1.0f / t.w);
+    f2 mfix = mk2(t.m.x / t.w, t.m.y / t.w);
     if (Centered<FORM>::value) {
       const f2 e = lum2(dfix, sfix) - kshift;
       mfix = mk2(fma_(-e.x, e.x, mfix.x), fma_(-e.y, e.y, mfix.y));
     }
     store_rec(out, i, dfix, sfix, mfix);
-  } else {
-    copy_rec(out, in, i);
   }
 }
 };
@@ -555,71 +562,63 @@ struct Dn32FastClampF {
 
 template <class Geo, int FORM>
 struct Dn32FallbackF {
+  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
   using R = typename DnT<FORM>::R;
   using N = typename DnT<FORM>::N;
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const N* __restrict__ len, const R* __restrict__ in, R* __restrict__ out) {
-  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
-  if (!inb(x, y, w, h)) return;
-  size_t i = (size_t)y * w + x;
-  float hl = ld_len(len, i);
-  float qmax = quad_max_len(len, x, y, w, h);
-  if (hl == 0.0f) {
-    store_rec(out, i, mk3(0.0f), mk3(0.0f), mk2(0.0f, 0.0f));
-    return;
-  }
-  hl = qmax;
-  f3 dd, sd;
-  f2 md;
+  __shared__ ShortStage<3> st;
+  const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
+  const bool inside = inb(x, y, w, h);
+  const size_t i = inside ? (size_t)y * w + x : 0;
+  const float own = inside ? ld_len(len, i) : 0.0f;
+  const float hl = inside ? quad_max_len(len, x, y, w, h) : 0.0f;
+  const bool is_short = own != 0.0f && hl < 4.0f * VLT_HISTORY_LEN_UNIT;
+  ShortPixel c = {mk3(0.0f), 0.0f, 0.0f, x, y, 1};
+  FilterSums<Centered<FORM>::value> t;
   f2 kshift = mk2(0.0f, 0.0f);  // centered form: the shift of the blended variances
-  if (hl < 4.0f * VLT_HISTORY_LEN_UNIT) {
-    EdgeStopFast es = make_es(geo.dep(i), geo.fwz(i) * 3.0f, 1.0f, geo.normal(i), 7);
-    float ws = 0.0f;
-    f3 dsum = mk3(0.0f), ssum = mk3(0.0f);
-    f2 msum = mk2(0.0f, 0.0f);
+  if (is_short) {
+    c.depth = geo.dep(i);
+    c.fz_sigma = 1.0f * (geo.fwz(i) * 3.0f);
+    c.normal = geo.normal(i);
     if (Centered<FORM>::value) {
       const Rec rc = load_rec(in, i);
       kshift = lum2(rc.d, rc.s);
     }
-    for (int oy = -3; oy <= 3; ++oy) {
-      for (int ox = -3; ox <= 3; ++ox) {
-        int cx = x + ox, cy = y + oy;
-        if (!(cx >= 0 && cy >= 0 && cx <= w - 1 && cy <= h - 1)) continue;
-        size_t j = (size_t)cy * w + cx;
-        float wt = es.weight(length2(mk2((float)ox, (float)oy)), geo.dep(j), geo.normal(j), mk2(0.0f, 0.0f)).x;
-        Rec r = load_rec(in, j);
-        ws = ws + wt;
-        dsum = fma3(wt, r.d, dsum);
-        ssum = fma3(wt, r.s, ssum);
-        if (Centered<FORM>::value) {
-          const f2 e = lum2(r.d, r.s) - kshift;
-          msum = mk2(fma_(wt, fma_(e.x, e.x, r.aux.x), msum.x), fma_(wt, fma_(e.y, e.y, r.aux.y), msum.y));
-        } else {
-          msum = mk2(fma_(wt, r.aux.x, msum.x), fma_(wt, r.aux.y, msum.y));
-        }
-      }
+  }
+  const auto finish = [&](f3 dd, f3 sd, f2 md) {
+    f2 var;
+    if (Centered<FORM>::value) {
+      // the long-history record holds the variance; the blend's is centered on kshift
+      const f2 e = is_short ? lum2(dd, sd) - kshift : mk2(0.0f, 0.0f);
+      var = mk2(fmax_(fma_(-e.x, e.x, md.x), 0.0f), fmax_(fma_(-e.y, e.y, md.y), 0.0f));
+    } else {
+      f2 fst = mk2(lum_fast(dd.x, dd.y, dd.z), lum_fast(sd.x, sd.y, sd.z));
+      var = mk2(fmax_(fma_(-fst.x, fst.x, md.x), 0.0f), fmax_(fma_(-fst.y, fst.y, md.y), 0.0f));
     }
-    float inv = 1.0f / ws;
-    dd = dsum * inv;
-    sd = ssum * inv;
-    md = msum * inv;
-  } else {
-    Rec r = load_rec(in, i);
-    dd = r.d;
-    sd = r.s;
-    md = r.aux;
+    float boost = fmax_(1.0f, (4.0f * VLT_HISTORY_LEN_UNIT) / hl);
+    store_rec(out, i, dd, sd, var * boost);
+  };
+  if (inside && !is_short) {
+    if (own == 0.0f) {
+      store_rec(out, i, mk3(0.0f), mk3(0.0f), mk2(0.0f, 0.0f));
+    } else {
+      const Rec r = load_rec(in, i);
+      finish(r.d, r.s, r.aux);
+    }
   }
-  f2 var;
-  if (Centered<FORM>::value) {
-    // the long-history record holds the variance; the blend's is centered on kshift
-    const bool blended = hl < 4.0f * VLT_HISTORY_LEN_UNIT;
-    const f2 e = blended ? lum2(dd, sd) - kshift : mk2(0.0f, 0.0f);
-    var = mk2(fmax_(fma_(-e.x, e.x, md.x), 0.0f), fmax_(fma_(-e.y, e.y, md.y), 0.0f));
-  } else {
-    f2 fst = mk2(lum_fast(dd.x, dd.y, dd.z), lum_fast(sd.x, sd.y, sd.z));
-    var = mk2(fmax_(fma_(-fst.x, fst.x, md.x), 0.0f), fmax_(fma_(-fst.y, fst.y, md.y), 0.0f));
+  filter_short_pixels<3>(
+      is_short, c, w, h, st,
+      [&](const ShortPixel& cc, size_t j, int ox, int oy) {
+        return short_weight(cc, geo, j, length2(mk2((float)ox, (float)oy)), 7);
+      },
+      [&](float wt, size_t j, bool ok) {
+        const Rec r = load_rec(in, j);
+        if (ok) t.add(wt, r, kshift);
+      });
+  if (is_short) {
+    const float inv = 1.0f / t.w;
+    finish(t.d * inv, t.s * inv, t.m * inv);
   }
-  float boost = fmax_(1.0f, (4.0f * VLT_HISTORY_LEN_UNIT) / hl);
-  store_rec(out, i, dd, sd, var * boost);
 }
 };
 
@@ -641,7 +640,6 @@ __device__ __forceinline__ void atrous_px(int x, int y, int w, int h, const Geo&
   size_t i = (size_t)y * w + x;
   Rec c = load_rec(in, i);
   EdgeStopFast es = make_es(geo.dep(i), geo.fwz(i), 1.0f, geo.normal(i), 7);
-  es.use_lumi = true;
   es.lumi_center = mk2(lum_fast(c.d.x, c.d.y, c.d.z), lum_fast(c.s.x, c.s.y, c.s.z));
   es.lumi_rcp = mk2((1.0f / fma_(4.0f, sqrt_(c.aux.x), 1e-8f)) * VLT_LOG2E,
                     (1.0f / fma_(4.0f, sqrt_(c.aux.y), 1e-8f)) * VLT_LOG2E);
