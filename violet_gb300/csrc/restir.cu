@@ -307,8 +307,7 @@ struct DiffTemporalF32F {
     }
     uint32_t rng = lcg_init_with_seed((uint32_t)x, (uint32_t)y, frame_rand);
     float w_sum = prev_w + new_w;
-    float chance = new_w / w_sum;
-    if (lcg_rand(rng) < chance) {
+    if (lcg_select(rng, new_w, w_sum)) {
       uint2 e = new_hpn[i];
       hp = hpn_pos(e.x, e.y);
       hn = hpn_normal(e.y);
@@ -370,8 +369,7 @@ struct DiffTemporalF {
     }
     uint32_t rng = lcg_init_with_seed((uint32_t)x, (uint32_t)y, frame_rand);
     float w_sum = prev_w + new_w;
-    float chance = new_w / w_sum;
-    if (lcg_rand(rng) < chance) {
+    if (lcg_select(rng, new_w, w_sum)) {
       uint2 e = new_hpn[i];
       h0 = e.x;
       h1 = e.y;
@@ -397,27 +395,31 @@ struct DiffSample {
 
 
 
-__device__ __forceinline__ DiffSample load_diff_rec(uint4 r, f3 pix_pos, f3 pix_n) {
+// Target function of a sample at a pixel; also the direction to it and its squared
+// distance.
+__device__ __forceinline__ void diff_target(DiffSample& s, f3 pix_pos, f3 pix_n, f3* dir, float* l2) {
+  const f3 v = s.pos - pix_pos;
+  *l2 = dot3(v, v);
+  *dir = v * rsqrt_(*l2);
+  s.tp = saturate(dot3(pix_n, *dir)) * luminance(s.rad);
+}
+
+__device__ __forceinline__ DiffSample load_diff(const uint4* p, size_t i, f3 pix_pos, f3 pix_n, f3* dir, float* l2) {
+  const uint4 r = p[i];
   DiffSample s;
   s.M = rsv_decode_M(r.x);
   s.W = rsv_decode_W(r.x);
   s.pos = hpn_pos(r.y, r.z);
   s.nrm = hpn_normal(r.z);
   s.rad = unpack_r11g11b10(r.w);
-  float nol = saturate(dot3(pix_n, normalize3(s.pos - pix_pos)));
-  s.tp = nol * luminance(s.rad);
+  diff_target(s, pix_pos, pix_n, dir, l2);
   return s;
 }
-
-__device__ __forceinline__ DiffSample load_diff(const uint4* p, size_t i, f3 pix_pos, f3 pix_n) {
-  return load_diff_rec(p[i], pix_pos, pix_n);
-}
 template <class CPtr>
-__device__ __forceinline__ DiffSample load_diff(CPtr p, size_t i, f3 pix_pos, f3 pix_n) {
+__device__ __forceinline__ DiffSample load_diff(CPtr p, size_t i, f3 pix_pos, f3 pix_n, f3* dir, float* l2) {
   DiffSample s;
   diff_load(p, i, &s.M, &s.W, &s.pos, &s.nrm, &s.rad, &s.bits);
-  float nol = saturate(dot3(pix_n, normalize3(s.pos - pix_pos)));
-  s.tp = nol * luminance(s.rad);
+  diff_target(s, pix_pos, pix_n, dir, l2);
   return s;
 }
 
@@ -446,7 +448,11 @@ __device__ __forceinline__ void store_empty_diff(DiffF16Ptr out, size_t i) {
 // adaptive radius, plane-distance test, Jacobian clamped to [0, 1]).
 template <class Geo, int FORM>
 struct DiffSpatialF {
-  static constexpr int kMinBlocks = 4;  // 64 registers: 8 tiles per SM (measured 7% faster)
+  // 48 registers, 10 tiles per SM. Two 1080p passes: 298 us with the selected sample and its
+  // quotient test in registers at 64, 285 us carrying its pixel, 273 us at 48 (f32 frame
+  // 1,562 -> 1,537 us, 3840x2160 f16 6,038 -> 5,935 us, reference-form block at 1280x720 168.7
+  // -> 161.9 us). Issue-bound: 1,868 warp instructions per 32 pixels at 70 % issue.
+  static constexpr int kMinBlocks = 5;
   static __device__ __forceinline__ void run(int x0, int y0, vlt_frame_params fp, int w, int h, DiffKnobs kn, Geo geo, const typename AoStore<FORM>::Filt* __restrict__ ao_tex, typename DiffStore<FORM>::CPtr in, typename DiffStore<FORM>::Ptr out, typename DiffStore<FORM>::Light* __restrict__ lighting, uint32_t frame_rand) {
   using S = DiffStore<FORM>;
   // The spiral's radius and angle offset of tap `it` depend only on it and the tap
@@ -476,8 +482,20 @@ struct DiffSpatialF {
   f3 pos = geo.pos(x, y, i);
   f3 nrm = geo.normal(i);
   float ao = load_ao(ao_tex, i);
-  DiffSample r = load_diff(in, i, pos, nrm);
-  float w_sum = r.W * r.tp * (float)r.M;
+  // Of the selected sample only its pixel is carried through the loop (the record is
+  // loaded again at the end): nine registers fewer than the decoded sample.
+  size_t sel = i;
+  uint32_t M;
+  float W, tp, w_sum;
+  {
+    f3 dir;
+    float l2;
+    const DiffSample c = load_diff(in, i, pos, nrm, &dir, &l2);
+    M = c.M;
+    W = c.W;
+    tp = c.tp;
+    w_sum = c.W * c.tp * (float)c.M;
+  }
   float radius = kn.radius_px > 0.0f ? kn.radius_px : (float)(w < h ? w : h) * 0.05f;
   radius = fmax_(radius * ao, 1.5f);
   uint32_t rng = lcg_init_with_seed((uint32_t)x, (uint32_t)y, frame_rand);
@@ -501,35 +519,37 @@ struct DiffSpatialF {
       radius = fmax_(radius * 0.5f, 1.5f);
       continue;
     }
-    DiffSample nb = load_diff(in, j, pos, nrm);
+    // rq = pos - nb.pos is the negated direction that the target function normalizes: its
+    // squared length and reciprocal root are the same numbers, and cos_rq the negated
+    // cosine (a zero's sign does not reach the result: the Jacobian is clamped at 0).
+    f3 dir;
+    float l2rq;
+    const DiffSample nb = load_diff(in, j, pos, nrm, &dir, &l2rq);
     f3 qq = pn - nb.pos;
-    f3 rq = pos - nb.pos;
     float l2qq = dot3(qq, qq);
-    float l2rq = dot3(rq, rq);
-    float cos_rq = dot3(nb.nrm, rq * rsqrt_(l2rq));
+    float cos_rq = -dot3(nb.nrm, dir);
     float cos_qq = dot3(nb.nrm, qq * rsqrt_(l2qq));
     float jac = (cos_rq / cos_qq) * (l2qq / l2rq);
     jac = clampf(jac, 0.0f, 10.0f);
     jac = clampf(jac, 0.0f, 1.0f);
     float tpn = nb.tp * jac;
     if (tpn <= 0.0f) continue;
-    nb.M = nb.M < 255u ? nb.M : 255u;
-    float wsn = nb.W * tpn * (float)nb.M;
+    const uint32_t nbM = nb.M < 255u ? nb.M : 255u;
+    float wsn = nb.W * tpn * (float)nbM;
     w_sum = w_sum + wsn;
-    float chance = wsn / w_sum;
-    if (lcg_rand(rng) < chance) {
-      r.nrm = nb.nrm;
-      r.pos = nb.pos;
-      r.rad = nb.rad;
-      r.tp = nb.tp;
-      r.bits = nb.bits;
+    if (lcg_select(rng, wsn, w_sum)) {
+      sel = j;
+      tp = nb.tp;
     }
-    r.M += nb.M;
+    M += nbM;
   }
-  if (r.tp > 0.0f) r.W = w_sum / (r.tp * (float)r.M);
+  f3 dir;
+  float l2;
+  DiffSample r = load_diff(in, sel, pos, nrm, &dir, &l2);
+  r.M = M;
+  r.W = tp > 0.0f ? w_sum / (tp * (float)M) : W;
   store_diff(out, i, r);
   if (lighting) {
-    f3 dir = normalize3(r.pos - pos);
     float nol = saturate(dot3(nrm, dir));
     f3 l = r.rad * (VLT_ONE_OVER_PI * nol * r.W);
     lighting[i] = S::light(l);
@@ -718,8 +738,7 @@ struct SpecTemporalF {
   }
   uint32_t rng = lcg_init_with_seed((uint32_t)x, (uint32_t)y, frame_rand);
   float w_sum = prev_w + new_w;
-  float chance_prev = prev_w / w_sum;
-  bool use_prev = lcg_rand(rng) < chance_prev;
+  const bool use_prev = lcg_select(rng, prev_w, w_sum);
   if (!use_prev) {
     rhp = nhp;
     rrad_bits = nrad_bits;
@@ -845,8 +864,7 @@ __device__ __forceinline__ void spec_spatial_px(int x, int y, vlt_frame_params f
       w_c = m_c * ctf * W;
     }
     float w_sum = w_c + w_nb;
-    float chance = w_nb / w_sum;
-    if (lcg_rand(rng) < chance) {
+    if (lcg_select(rng, w_nb, w_sum)) {
       hit = hitn;
       rad = radn;
       rad_bits = radn_bits;

@@ -408,6 +408,21 @@ VLT_HD uint32_t lcg_xorshift(uint32_t& x) {
 }
 VLT_HD float lcg_rand(uint32_t& s) { return lcg_uint_to_float(lcg_xorshift(s)); }
 
+// lcg_rand(s) < RN(a / b), the resampling passes' selection, mostly without the division.
+// The draw t is a multiple of 2^-23 below 1, so RN(a / b) > t holds where a / b exceeds t
+// by 2^-24 or more and fails where a / b <= t; d = RN(a - t b) has the sign of a - t b and
+// decides both (the threshold b 2^-22 leaves room for its rounding). Only what lies
+// between, and divisors that are small, negative or NaN, takes the quotient.
+VLT_HD bool lcg_select(uint32_t& s, float a, float b) {
+  const float t = lcg_rand(s);
+  const float d = fma_(-t, b, a);
+  if (b >= 0x1p-100f) {
+    if (d <= 0.0f) return false;
+    if (d > b * 0x1p-22f) return true;
+  }
+  return t < a / b;
+}
+
 // Un-seeded XXHash32 variant of rand.hlsl:82-112.
 VLT_HD uint32_t rotl32(uint32_t h, int r) { return (h << r) | (h >> (32 - r)); }
 struct XXHash32 {
