@@ -17,7 +17,8 @@ LIB = os.path.join(OUT_DIR, "libvlt.so")
 
 SOURCES = ["restir.cu", "denoise.cu", "denoise_f32.cu", "hashgrid.cu", "trace.cu", "post.cu", "scene.cu", "launch.cu", "api.cu", "batch.cu", "server.cu"]
 HEADERS = ["vlt_math.cuh", "vlt_device.cuh", "vlt_launch.cuh", "vlt_internal.h", "brdf.cuh", "scene_gen.cuh", "trace.cuh",
-           "hashgrid.cuh", "vlt_compact.cuh", "short_history.cuh"]
+           "hashgrid.cuh", "vlt_compact.cuh", "short_history.cuh",
+           "exact_math.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_103a,code=sm_103a",

@@ -27,8 +27,10 @@ __device__ __forceinline__ f3 f_schlick(float u, f3 f0) {
   return mk3(f + f0.x * (1.0f - f), f + f0.y * (1.0f - f), f + f0.z * (1.0f - f));
 }
 
-// ggx_brdf_integral_approx (brdf.hlsl:180-199) [Hirvonen 2019].
-__device__ __forceinline__ f3 ggx_integral(float nov, float roughness, f3 f0) {
+// ggx_brdf_integral_approx (brdf.hlsl:180-199) [Hirvonen 2019]. For nov and roughness in
+// [0, 1] both denominators lie in [1, 2000].
+template <class A>
+__device__ __forceinline__ f3 ggx_integral(A& ar, float nov, float roughness, f3 f0) {
   float a = roughness * roughness;
   float a2 = a * a;
   float a3 = a * a2;
@@ -41,15 +43,21 @@ __device__ __forceinline__ f3 ggx_integral(float nov, float roughness, f3 f0) {
   float m1x = 1.0f * 1.0f + 2.92338f * c + 59.4188f * c3;
   float m1y = 20.3225f * 1.0f + -27.0302f * c + 222.592f * c3;
   float m1z = 121.563f * 1.0f + 626.13f * c + 316.627f * c3;
-  k0 = k0 / (1.0f * m1x + a * m1y + a3 * m1z);
+  ar.see(fabs_(k0));
+  k0 = A::div(k0, 1.0f * m1x + a * m1y + a3 * m1z);
   float m2x = 0.0365463f * 1.0f + 3.32707f * c;
   float m2y = 9.0632f * 1.0f + -9.04756f * c;
   float k1 = 1.0f * m2x + a * m2y;
   float m3x = 1.0f * 1.0f + 3.59685f * c2 + -1.36772f * c3;
   float m3y = 9.04401f * 1.0f + -16.3174f * c2 + 9.22949f * c3;
   float m3z = 5.56589f * 1.0f + 19.7886f * c2 + -20.2123f * c3;
-  k1 = k1 / (1.0f * m3x + a * m3y + a3 * m3z);
+  ar.see(fabs_(k1));
+  k1 = A::div(k1, 1.0f * m3x + a * m3y + a3 * m3z);
   return mk3(k0 + k1 * f0.x, k0 + k1 * f0.y, k0 + k1 * f0.z);
+}
+__device__ __forceinline__ f3 ggx_integral(float nov, float roughness, f3 f0) {
+  Ieee ar;
+  return ggx_integral(ar, nov, roughness, f0);
 }
 
 // vis_smith_G2_height_correlated_GGX, optimized form (brdf.hlsl:99-113).

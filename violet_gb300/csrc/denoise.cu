@@ -82,7 +82,7 @@ struct DnTemporalF {
     return;
   }
   const float bw = (float)w, bh = (float)h;
-  f2 screen_uv = mk2(((float)x + 0.5f) / bw, ((float)y + 0.5f) / bh);
+  f2 screen_uv = pixel_uv(x, y, w, h);
   const f3 gnormal = geo.normal(i);
   const float grough = geo.rough(i);
   const float fwz = geo.fwz(i);
@@ -541,16 +541,6 @@ __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 // A factor of 1 that only the host knows, a kernel argument, keeps the two apart.
 __device__ __forceinline__ float2 madd2(float2 a, float2 b, float2 c, float one) {
   return __ffma2_rn(__fmul2_rn(a, b), bc2(one), c);
-}
-
-// a / b, correctly rounded, from r = RN(1 / b): q = RN(a r), then one correction by the
-// exact remainder (Markstein 1990). An exhaustive comparison over all 2^46 pairs of
-// binary32 mantissas found no difference from the IEEE quotient; the remainder must
-// not underflow, so a is 0 or of magnitude at least 2^-100 while b is of ordinary size
-// (|b| in [2^-30, 2^40] here), or the quotient of a smaller a may be off by an ulp.
-__device__ __forceinline__ float div_shared(float a, float b, float r) {
-  const float q = a * r;
-  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
 
 struct AtrousOut {

@@ -250,7 +250,7 @@ struct Dn32TemporalF {
     return;
   }
   const float bw = (float)w, bh = (float)h;
-  f2 screen_uv = mk2(((float)x + 0.5f) / bw, ((float)y + 0.5f) / bh);
+  f2 screen_uv = pixel_uv(x, y, w, h);
   const f3 gnormal = geo.normal(i);
   const float grough = geo.rough(i);
   const float fwz = geo.fwz(i);

@@ -82,7 +82,7 @@ struct AoGenF {
   f4 hr = mul44(fp.prev_view_proj, mk4(position.x, position.y, position.z, 1.0f));
   f2 ndc_r = mk2(hr.x / hr.w - fp.jitter[2], hr.y / hr.w - fp.jitter[3]);
   f2 mv = mk2((ndc.x - ndc_r.x) * 0.5f, (ndc.y - ndc_r.y) * 0.5f);
-  f2 src_uv = mk2(((float)x + 0.5f) / (float)w, ((float)y + 0.5f) / (float)h);
+  f2 src_uv = pixel_uv(x, y, w, h);
   f2 huv = mk2(src_uv.x - mv.x, src_uv.y - mv.y);
   float hx = 0.0f, ha = 0.0f;
   bool in_last = huv.x == saturate(huv.x) && huv.y == saturate(huv.y);
@@ -563,42 +563,68 @@ struct DiffSpatialF {
 // calc_things (ind_spec_temporal_resample.hlsl:63-144) == SpecTragetFunction::on_sample
 // (ind_spec_spatial_resample.hlsl:69-151), split into the part that depends only on
 // the shading point (view direction, NoV, Smith terms of V) and the per-sample part.
+// A: the arithmetic policy (exact_math.cuh). Ranges that hold by construction: the
+// roughness is in [0.002, 1] (decoded values in [0, 1]), the clamped cosines in [0, 1], so
+// the radicands of the Smith terms are in [4e-6, 2], the GGX denominator in [4e-6, 2] and
+// lp in [0.001, 1]; a zero nov or nol makes g 0 whatever its quotients gave.
+template <class A>
 struct SpecTarget {
   f3 pos, n, f0, v;
   float roughness, r2, nov, lp, kv;
 
-  __device__ __forceinline__ void init(f3 view_pos, f3 p, f3 nn, float pr, f3 f0v) {
+  __device__ __forceinline__ void init(A& ar, f3 view_pos, f3 p, f3 nn, float pr, f3 f0v) {
     pos = p;
     n = nn;
     f0 = f0v;
     roughness = fmax_(pr * pr, 0.002f);
     r2 = roughness * roughness;
-    v = normalize3(view_pos - p);
+    const f3 d = view_pos - p;
+    const float d2 = dot3(d, d);
+    ar.see(d2);
+    v = d * A::rsqrt(d2);
     nov = saturate(dot3(n, v));
-    lp = lambda_pomc(nov, roughness);
-    kv = g_k(nov, r2);
+    ar.see_unless(nov == 0.0f, nov);
+    const float sq = A::sqrt((-r2 * nov + nov) * nov + r2);
+    lp = (nov + sq) / 2.0f;   // lambda_pomc
+    kv = A::div(sq, nov);     // g_k
+  }
+  // (1 + kv) / (kv + g_k(nol)), 0 where either cosine is 0.
+  __device__ __forceinline__ float smith(A& ar, float nol) const {
+    ar.see_unless(nol == 0.0f, nol);
+    float g = A::div(1.0f + kv, kv + A::div(A::sqrt((-r2 * nol + nol) * nol + r2), nol));
+    if (nol <= 0.0f) g = 0.0f;
+    if (nov <= 0.0f) g = 0.0f;
+    return g;
+  }
+  // 0.25 d_ggx / lp
+  __device__ __forceinline__ float vndf(float noh) const {
+    const float a = noh * roughness;
+    const float k = A::div(roughness, 1.0f - noh * noh + a * a);
+    return A::div(0.25f * (k * k * VLT_ONE_OVER_PI), lp);
   }
   // source pdf and luminance(radiance * brdf_NoL_over_source_pdf) * pdf.
-  __device__ __forceinline__ void eval(f3 hit, f3 rad, float* source_pdf, float* tf, float* w) const {
-    f3 l = normalize3(hit - pos);
-    f3 hv = normalize3(v + l);
+  __device__ __forceinline__ void eval(A& ar, f3 hit, f3 rad, float* source_pdf, float* tf, float* w) const {
+    const f3 dl = hit - pos;
+    const float l2 = dot3(dl, dl);
+    ar.see(l2);
+    const f3 l = dl * A::rsqrt(l2);
+    const f3 dh = v + l;
+    const float h2 = dot3(dh, dh);
+    ar.see(h2);
+    const f3 hv = dh * A::rsqrt(h2);
     float noh = saturate(dot3(n, hv));
-    float D = d_ggx(noh, roughness);
-    float sp = 0.25f * D / lp;
+    float sp = vndf(noh);
     float nol = saturate(dot3(n, l));
     float loh = saturate(dot3(l, hv));
     f3 F = f_schlick(loh, f0);
-    float g = (1.0f + kv) / (kv + g_k(nol, r2));
-    if (nol <= 0.0f) g = 0.0f;
-    if (nov <= 0.0f) g = 0.0f;
-    float ww = luminance(rad * (F * g));
+    float ww = luminance(rad * (F * smith(ar, nol)));
     *source_pdf = sp;
     *w = ww;
     *tf = ww * sp;
   }
-  __device__ __forceinline__ float tf(f3 hit, f3 rad) const {
+  __device__ __forceinline__ float tf(A& ar, f3 hit, f3 rad) const {
     float sp, t, ww;
-    eval(hit, rad, &sp, &t, &ww);
+    eval(ar, hit, rad, &sp, &t, &ww);
     return t;
   }
 };
@@ -717,19 +743,20 @@ struct SpecTemporalF {
   float rough = geo.rough(i);
   uint32_t mmax = f2u_rz((float)m_cap * rough);
   M = M < mmax ? M : mmax;
-  SpecTarget cur;
-  cur.init(vpos3(fp.view_pos), pos, geo.normal(i), rough, geo.f0(i));
+  Ieee ar;
+  SpecTarget<Ieee> cur;
+  cur.init(ar, vpos3(fp.view_pos), pos, geo.normal(i), rough, geo.f0(i));
   float sp_new, new_tf, new_w;
-  cur.eval(nhp, nrad, &sp_new, &new_tf, &new_w);
+  cur.eval(ar, nhp, nrad, &sp_new, &new_tf, &new_w);
   float prev_w = W * (rtf * (float)M);
   if (M > 0) {
-    SpecTarget prv;
-    prv.init(vpos3(fp.prev_view_pos), pos, pn, prough, pf0);
-    float ptoc = prv.tf(nhp, nrad);
+    SpecTarget<Ieee> prv;
+    prv.init(ar, vpos3(fp.prev_view_pos), pos, pn, prough, pf0);
+    float ptoc = prv.tf(ar, nhp, nrad);
     float curr_m = new_tf / (new_tf + ptoc * (float)M);
     if (new_tf == 0.0f) curr_m = 0.0f;
     new_w = curr_m * new_w;
-    float ctop = cur.tf(rhp, rrad);
+    float ctop = cur.tf(ar, rhp, rrad);
     float m_num = rtf * (float)M;
     float prev_m = m_num / (m_num + ctop);
     if (m_num == 0.0f) prev_m = 0.0f;
@@ -790,9 +817,10 @@ struct SpecLight<FORM_F16> {
   using T = uint2;  // half4 {rgb, ray length}
 };
 
-// One pixel of the specular spatial pass (the pixel (x, y) is inside the image).
-template <class Geo, int FORM>
-__device__ __forceinline__ void spec_spatial_px(int x, int y, vlt_frame_params fp, int w, int h, SpecKnobs kn, Geo geo, typename SpecStore<FORM>::CPtr in, typename SpecLight<FORM>::T* __restrict__ lighting, uint16_t* __restrict__ ray_len_out, typename SpecStore<FORM>::Ptr out, uint32_t frame_rand) {
+// One pixel of the specular spatial pass (the pixel (x, y) is inside the image), over an
+// arithmetic policy; returns false, having stored nothing, where that was left.
+template <class A, class Geo, int FORM>
+__device__ __forceinline__ bool spec_spatial_px_as(int x, int y, const vlt_frame_params& fp, int w, int h, const SpecKnobs& kn, const Geo& geo, const typename SpecStore<FORM>::CPtr& in, typename SpecLight<FORM>::T* __restrict__ lighting, uint16_t* __restrict__ ray_len_out, const typename SpecStore<FORM>::Ptr& out, uint32_t frame_rand) {
   size_t i = (size_t)y * w + x;
   float depth = geo.dep(i);
   if (depth == 0.0f) {
@@ -803,13 +831,14 @@ __device__ __forceinline__ void spec_spatial_px(int x, int y, vlt_frame_params f
       z.W = 0.0f;
       spec_st(out, i, z);
     }
-    return;
+    return true;
   }
+  A ar;
   f3 pos = geo.pos(x, y, i);
   const f3 view_pos = vpos3(fp.view_pos);
   float prc = geo.rough(i);
-  SpecTarget center;
-  center.init(view_pos, pos, geo.normal(i), prc, geo.f0(i));
+  SpecTarget<A> center;
+  center.init(ar, view_pos, pos, geo.normal(i), prc, geo.f0(i));
   const SpecSample c0 = spec_ld(in, x, y, w, h);
   uint32_t M = c0.M;
   float W = c0.W;
@@ -823,7 +852,8 @@ __device__ __forceinline__ void spec_spatial_px(int x, int y, vlt_frame_params f
   for (uint32_t it = 0; it < n_iter; ++it) {
     float u0 = lcg_rand(rng);
     float u1 = lcg_rand(rng);
-    float rr = sqrt_(u0);
+    ar.see(u0);
+    float rr = A::sqrt(u0);
     float s, c;
     sincos_(VLT_TWO_PI * u1, &s, &c);
     float ox = rr * c, oy = rr * s;
@@ -852,28 +882,64 @@ __device__ __forceinline__ void spec_spatial_px(int x, int y, vlt_frame_params f
     float tfn = nb.tf;
     float w_nb, w_c;
     {
-      float ctf_on_n = center.tf(hitn, radn);
-      float m_nb = (tfn * (float)Mn) / (tfn * (float)Mn + ctf_on_n * (float)M);
-      if (tfn * (float)Mn == 0.0f) m_nb = 0.0f;
+      float ctf_on_n = center.tf(ar, hitn, radn);
+      const float a_nb = tfn * (float)Mn, b_nb = a_nb + ctf_on_n * (float)M;
+      ar.see_unless(a_nb == 0.0f, a_nb);
+      ar.see_unless(a_nb == 0.0f, b_nb);
+      float m_nb = A::div(a_nb, b_nb);
+      if (a_nb == 0.0f) m_nb = 0.0f;
       w_nb = m_nb * tfn * Wn;
-      SpecTarget nbt;
-      nbt.init(view_pos, pn, nn, geo.rough(j), geo.f0(j));
-      float ntf_on_c = nbt.tf(hit, rad);
-      float m_c = (ctf * (float)M) / (ctf * (float)M + ntf_on_c * (float)Mn);
-      if (ctf * (float)M == 0.0f) m_c = 0.0f;
+      SpecTarget<A> nbt;
+      nbt.init(ar, view_pos, pn, nn, geo.rough(j), geo.f0(j));
+      float ntf_on_c = nbt.tf(ar, hit, rad);
+      const float a_c = ctf * (float)M, b_c = a_c + ntf_on_c * (float)Mn;
+      ar.see_unless(a_c == 0.0f, a_c);
+      ar.see_unless(a_c == 0.0f, b_c);
+      float m_c = A::div(a_c, b_c);
+      if (a_c == 0.0f) m_c = 0.0f;
       w_c = m_c * ctf * W;
     }
     float w_sum = w_c + w_nb;
-    if (lcg_select(rng, w_nb, w_sum)) {
+    ar.see_unless(w_sum == 0.0f, w_sum);
+    if (ar.select(rng, w_nb, w_sum)) {
       hit = hitn;
       rad = radn;
       rad_bits = radn_bits;
       ctf = tfn;
     }
     M += Mn;
-    W = ctf > 0.0f ? w_sum / ctf : 0.0f;
+    ar.see_unless(!(ctf > 0.0f), ctf);  // a zero sum divided by a positive number is that zero
+    W = ctf > 0.0f ? (w_sum == 0.0f ? w_sum : A::div(w_sum, ctf)) : 0.0f;
   }
-  float ray_len = length3(hit - pos);
+  const f3 dl = hit - pos;
+  const float l2 = dot3(dl, dl);
+  ar.see(l2);
+  const float ray_len = A::sqrt(l2);
+  f3 li = mk3(0.0f);
+  if (lighting) {
+    const f3 l = dl * A::rcp(ray_len);
+    const f3 dh = center.v + l;
+    const float h2 = dot3(dh, dh);
+    ar.see(h2);
+    const f3 hv = dh * A::rsqrt(h2);
+    float nol = saturate(dot3(center.n, l));
+    float noh = saturate(dot3(center.n, hv));
+    float loh = saturate(dot3(l, hv));
+    f3 F = f_schlick(loh, center.f0);
+    float vndf = center.vndf(noh);
+    float gg = center.smith(ar, nol);
+    li = rad * ((F * gg) * (vndf * W));
+    f3 refl = ggx_integral(ar, center.nov, center.roughness, center.f0);
+    refl = mk3(fmax_(refl.x, 1.0f / 65536.0f), fmax_(refl.y, 1.0f / 65536.0f), fmax_(refl.z, 1.0f / 65536.0f));
+    ar.see(refl.x);
+    ar.see(refl.y);
+    ar.see(refl.z);
+    ar.see_unless(li.x == 0.0f, li.x);
+    ar.see_unless(li.y == 0.0f, li.y);
+    ar.see_unless(li.z == 0.0f, li.z);
+    li = mk3(A::div(li.x, refl.x), A::div(li.y, refl.y), A::div(li.z, refl.z));
+  }
+  if (!ar.ok()) return false;
   if (spec_has(out)) {
     SpecSample o;
     o.M = M;
@@ -885,27 +951,26 @@ __device__ __forceinline__ void spec_spatial_px(int x, int y, vlt_frame_params f
     spec_st(out, i, o);
   }
   if (lighting) {
-    const float roughness = center.roughness;
-    f3 l = normalize3(hit - pos);
-    f3 hv = normalize3(center.v + l);
-    float nol = saturate(dot3(center.n, l));
-    float nov = center.nov;
-    float noh = saturate(dot3(center.n, hv));
-    float loh = saturate(dot3(l, hv));
-    f3 F = f_schlick(loh, center.f0);
-    float D = d_ggx(noh, roughness);
-    float vndf = 0.25f * D / center.lp;
-    float gg = (1.0f + center.kv) / (center.kv + g_k(nol, center.r2));
-    if (nol <= 0.0f) gg = 0.0f;
-    if (nov <= 0.0f) gg = 0.0f;
-    f3 li = rad * ((F * gg) * (vndf * W));
-    f3 refl = ggx_integral(nov, roughness, center.f0);
-    refl = mk3(fmax_(refl.x, 1.0f / 65536.0f), fmax_(refl.y, 1.0f / 65536.0f), fmax_(refl.z, 1.0f / 65536.0f));
-    li = li / refl;
     store_spec_light(lighting, ray_len_out, i, li, ray_len);
   } else if (ray_len_out) {
     ray_len_out[i] = (uint16_t)f32tof16(ray_len);
   }
+  return true;
+}
+
+// One in some 10^6 pixels leaves the range (a draw within 2^-22 of its quotient, a draw of
+// 0) and is computed again with the IEEE operations. The tap chain's latency bounds the
+// pass: about twenty IEEE divisions and roots per tap, each the end of a basic block, kept
+// the two target functions of a tap from overlapping. Over Ranged the instruction count
+// stays (the range tests cost what the shorter forms save, 40.3 M for a 960x540 pass) at 64
+// instead of 58 % issue: 1920x1080 f32 frame 1,538 -> 1,507 us, 3840x2160 f16 frame 5,931 ->
+// 5,811 us, the per-pass entries at 1920x1080 (temporal and spatial, with the raw
+// G-buffer's cheaper decode) 252 -> 230 us. The diffuse spatial pass, which is bound by
+// issue, got slower over it (1280x720 156 -> 166 us at 48 registers, 155 at 64).
+template <class Geo, int FORM>
+__device__ __forceinline__ void spec_spatial_px(int x, int y, const vlt_frame_params& fp, int w, int h, const SpecKnobs& kn, const Geo& geo, const typename SpecStore<FORM>::CPtr& in, typename SpecLight<FORM>::T* __restrict__ lighting, uint16_t* __restrict__ ray_len_out, const typename SpecStore<FORM>::Ptr& out, uint32_t frame_rand) {
+  if (!spec_spatial_px_as<Ranged, Geo, FORM>(x, y, fp, w, h, kn, geo, in, lighting, ray_len_out, out, frame_rand))
+    spec_spatial_px_as<Ieee, Geo, FORM>(x, y, fp, w, h, kn, geo, in, lighting, ray_len_out, out, frame_rand);
 }
 
 // ind_spec_spatial_resample.hlsl:169-448, per tile. The tap count of a pixel is
@@ -968,6 +1033,7 @@ __global__ void __launch_bounds__(32 * NW, 32 / NW)  // 64 registers
                           typename SpecLight<FORM>::T* __restrict__ lighting, uint16_t* __restrict__ ray_len_out,
                           typename SpecStore<FORM>::Ptr out, uint32_t frame_rand) {
   constexpr int NT = 32 * NW;
+  static_assert(NT <= kMaxThreads, "SortedRounds holds two pixels of up to kMaxThreads threads");
   __shared__ SortedRounds sr;
   const int x0 = (int)blockIdx.x * 32, y0 = (int)blockIdx.y * 2 * NW;
   const int tid = (int)threadIdx.x;

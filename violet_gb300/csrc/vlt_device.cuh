@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "../../include/vlt.h"
+#include "exact_math.cuh"
 #include "vlt_math.cuh"
 
 namespace vlt {
@@ -56,11 +57,24 @@ __device__ __forceinline__ f2 ld_half2(const uint32_t* __restrict__ p, int x, in
 
 __device__ __forceinline__ uint32_t pack_half2(f2 v) { return f32tof16(v.x) | (f32tof16(v.y) << 16); }
 
+// (pixel + 0.5) / size: operands in [0.5, 16384].
+__device__ __forceinline__ f2 pixel_uv(int x, int y, int w, int h) {
+  return mk2(div_ranged((float)x + 0.5f, (float)w), div_ranged((float)y + 0.5f, (float)h));
+}
+
 // cs_depth_to_position (frame_bindings.hlsl:57-61) with an explicit matrix.
 __device__ __forceinline__ f3 depth_to_position(const float* inv_vp, int x, int y, int w, int h, float depth) {
-  float u = ((float)x + 0.5f) / (float)w;
-  float v = ((float)y + 0.5f) / (float)h;
-  f4 p = mul44(inv_vp, mk4(u * 2.0f - 1.0f, v * 2.0f - 1.0f, depth, 1.0f));
+  const f2 uv = pixel_uv(x, y, w, h);
+  f4 p = mul44(inv_vp, mk4(uv.x * 2.0f - 1.0f, uv.y * 2.0f - 1.0f, depth, 1.0f));
+  Ranged r;
+  r.see(fabs_(p.w));
+  r.see(fabs_(p.x));
+  r.see(fabs_(p.y));
+  r.see(fabs_(p.z));
+  if (r.ok()) {
+    const float rw = rcp_ranged(p.w);
+    return mk3(div_shared(p.x, p.w, rw), div_shared(p.y, p.w, rw), div_shared(p.z, p.w, rw));
+  }
   return mk3(p.x / p.w, p.y / p.w, p.z / p.w);
 }
 
