@@ -1130,20 +1130,19 @@ static vlt_status frame_run_impl(vlt_view* v, const vlt_frame_inputs* in, const 
     float4* rsrc = b.rec[4];
     float4* rdst = b.rec[2];
     const uint32_t iters = P.atrous_iterations;
-    // f16 form: the iterations between the first and the last keep f32 records
-    // (atr32); the last record, read by the final lighting or the next traced frame,
-    // is the form's own (rec[3]).
-    bool src_f32 = false;
+    // The iterations between the first and the last keep interleaved f32 records (in the
+    // f16 form in atr32); the last record, read by the final lighting or the next traced
+    // frame, is the form's own (rec[3] in the f16 form).
+    bool src_mid = false;
     for (uint32_t k = 0; k < iters; ++k) {
       bool last = k + 1 == iters;
       void* od = last && out ? out->diffuse : nullptr;
       void* os = last && out ? out->specular : nullptr;
-      const bool dst_f32 = f16 && !last;
       if (f16) rdst = last ? b.rec[3] : b.atr32[k & 1];
       void* ro = last && !keep_den ? nullptr : (void*)rdst;
-      STAGE("dn_atrous", launch_dn32_atrous(exd, form, w, h, ga, rsrc, ro, od, os, 1 << k, src_f32, dst_f32));
+      STAGE("dn_atrous", launch_dn32_atrous(exd, form, w, h, ga, rsrc, ro, od, os, (int)k, src_mid, !last));
       rsrc = rdst;
-      src_f32 = dst_f32;
+      src_mid = !last;
       if (!f16) rdst = rdst == b.rec[2] ? b.rec[3] : b.rec[2];
     }
     den = keep_den ? (const void*)rsrc : nullptr;
