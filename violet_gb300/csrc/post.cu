@@ -86,7 +86,7 @@ struct FinalLightingF {
 namespace {
 
 // Mitchell-Netravali filter, B = C = 1/3 (temporal_aa.hlsl `mitchell`).
-__device__ __forceinline__ float mitchell(float x) {
+VLT_HD float mitchell(float x) {
   const float B = 1.0f / 3.0f, Cc = 1.0f / 3.0f;
   float y = 0.0f;
   float x2 = x * x;
@@ -110,6 +110,21 @@ __device__ __forceinline__ f3 clip_aabb(f3 c, f3 half_ext, f3 q) {
   return q;
 }
 
+// The source filter's weight of the neighbour at (dx, dy) - (1, 1): the sample's offset
+// from the pixel depends on the jitter alone, so that nine weights serve the image. They
+// are computed on the host in the same binary32 operations (each pixel took nine square
+// roots and divisions for them: 50 -> 35 us at 1280x720 in the reference form).
+struct TaaWeights {
+  float w[3][3];
+};
+TaaWeights taa_weights(const vlt_frame_params& fp, int w, int h) {
+  const float sox = -fp.jitter[0] * 0.5f * (float)w, soy = -fp.jitter[1] * 0.5f * (float)h;
+  TaaWeights t;
+  for (int dx = 0; dx < 3; ++dx)
+    for (int dy = 0; dy < 3; ++dy) t.w[dx][dy] = mitchell(length2(mk2((float)(dx - 1) + sox, (float)(dy - 1) + soy)));
+  return t;
+}
+
 }  // namespace
 
 // temporal_aa.hlsl `main`: Mitchell-filtered 3x3 source, bilinear history at the
@@ -120,24 +135,25 @@ template <int FORM>
 struct TaaF {
   using C = ColorIO<FORM>;
   using T = typename C::T;
-  static __device__ __forceinline__ void run(int x0, int y0, vlt_frame_params fp, int w, int h,
+  static __device__ __forceinline__ void run(int x0, int y0, vlt_frame_params fp, int w, int h, TaaWeights tw,
                                              const float* __restrict__ depth, const T* __restrict__ source,
                                              const T* __restrict__ history, T* __restrict__ out_hist,
                                              T* __restrict__ out_user, uint32_t has_history) {
     int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
     if (!inb(x, y, w, h)) return;
     size_t i = (size_t)y * w + x;
-    const float sox = -fp.jitter[0] * 0.5f * (float)w, soy = -fp.jitter[1] * 0.5f * (float)h;
     f3 accu = mk3(0.0f), nmin = mk3(1e5f), nmax = mk3(-1e5f), m1 = mk3(0.0f), m2 = mk3(0.0f);
     float wsum = 0.0f;
+#pragma unroll
     for (int dx = -1; dx <= 1; ++dx) {
+#pragma unroll
       for (int dy = -1; dy <= 1; ++dy) {
-        int px = x + dx, py = y + dy;
-        px = px < 0 ? 0 : (px > w - 1 ? w - 1 : px);
-        py = py < 0 ? 0 : (py > h - 1 ? h - 1 : py);
-        f2 off = mk2((float)(px - x) + sox, (float)(py - y) + soy);
+        // a tap beyond the edge is the edge pixel with the edge pixel's offset
+        const bool ox = x + dx < 0 || x + dx > w - 1, oy = y + dy < 0 || y + dy > h - 1;
+        const int px = ox ? x : x + dx, py = oy ? y : y + dy;
         f3 nb = C::ld(source, (size_t)py * w + px);
-        float wt = mitchell(length2(off));
+        const float wx = oy ? tw.w[dx + 1][1] : tw.w[dx + 1][dy + 1], wc = oy ? tw.w[1][1] : tw.w[1][dy + 1];
+        const float wt = ox ? wc : wx;
         accu = accu + nb * wt;
         wsum = wsum + wt;
         nmin = min3v(nmin, nb);
@@ -149,11 +165,11 @@ struct TaaF {
     f3 src = accu / wsum;
     f3 pos = depth_to_position(fp.inv_view_proj, x, y, w, h, depth[i]);
     f4 hp = mul44(fp.view_proj, mk4(pos.x, pos.y, pos.z, 1.0f));
-    f2 ndc = mk2(hp.x / hp.w - fp.jitter[0], hp.y / hp.w - fp.jitter[1]);
+    f2 ndc = perspective_xy(hp) - mk2(fp.jitter[0], fp.jitter[1]);
     f4 hr = mul44(fp.prev_view_proj, mk4(pos.x, pos.y, pos.z, 1.0f));
-    f2 ndc_r = mk2(hr.x / hr.w - fp.jitter[2], hr.y / hr.w - fp.jitter[3]);
+    f2 ndc_r = perspective_xy(hr) - mk2(fp.jitter[2], fp.jitter[3]);
     f2 mv = mk2((ndc.x - ndc_r.x) * 0.5f, (ndc.y - ndc_r.y) * 0.5f);
-    f2 huv = mk2(((float)x + 0.5f) / (float)w - mv.x, ((float)y + 0.5f) / (float)h - mv.y);
+    const f2 huv = pixel_uv(x, y, w, h) - mv;
     bool out_of_view = huv.x != saturate(huv.x) || huv.y != saturate(huv.y);
     f3 result;
     if (out_of_view || !has_history) {
@@ -205,7 +221,8 @@ void launch_final_lighting(const Exec& ex, int form, const vlt_frame_params& fp,
 
 void launch_taa(const Exec& ex, int form, const vlt_frame_params& fp, int w, int h, const float* depth,
                 const void* source, const void* history, void* out_hist, void* out_user, uint32_t has_history) {
-  VLT_POST_FORM(form, (launch2d<TaaF<F>>(ex, "taa", w, h, fp, w, h, depth, (const typename ColorIO<F>::T*)source,
+  const TaaWeights tw = taa_weights(fp, w, h);
+  VLT_POST_FORM(form, (launch2d<TaaF<F>>(ex, "taa", w, h, fp, w, h, tw, depth, (const typename ColorIO<F>::T*)source,
                                          (const typename ColorIO<F>::T*)history, (typename ColorIO<F>::T*)out_hist,
                                          (typename ColorIO<F>::T*)out_user, has_history)));
 }

@@ -62,20 +62,35 @@ __device__ __forceinline__ f2 pixel_uv(int x, int y, int w, int h) {
   return mk2(div_ranged((float)x + 0.5f, (float)w), div_ranged((float)y + 0.5f, (float)h));
 }
 
+// h.xyz / h.w and h.xy / h.w: one reciprocal where every operand allows it.
+__device__ __forceinline__ f3 perspective(f4 h) {
+  Ranged r;
+  r.see(fabs_(h.w));
+  r.see(fabs_(h.x));
+  r.see(fabs_(h.y));
+  r.see(fabs_(h.z));
+  if (r.ok()) {
+    const float rw = rcp_ranged(h.w);
+    return mk3(div_shared(h.x, h.w, rw), div_shared(h.y, h.w, rw), div_shared(h.z, h.w, rw));
+  }
+  return mk3(h.x / h.w, h.y / h.w, h.z / h.w);
+}
+__device__ __forceinline__ f2 perspective_xy(f4 h) {
+  Ranged r;
+  r.see(fabs_(h.w));
+  r.see(fabs_(h.x));
+  r.see(fabs_(h.y));
+  if (r.ok()) {
+    const float rw = rcp_ranged(h.w);
+    return mk2(div_shared(h.x, h.w, rw), div_shared(h.y, h.w, rw));
+  }
+  return mk2(h.x / h.w, h.y / h.w);
+}
+
 // cs_depth_to_position (frame_bindings.hlsl:57-61) with an explicit matrix.
 __device__ __forceinline__ f3 depth_to_position(const float* inv_vp, int x, int y, int w, int h, float depth) {
   const f2 uv = pixel_uv(x, y, w, h);
-  f4 p = mul44(inv_vp, mk4(uv.x * 2.0f - 1.0f, uv.y * 2.0f - 1.0f, depth, 1.0f));
-  Ranged r;
-  r.see(fabs_(p.w));
-  r.see(fabs_(p.x));
-  r.see(fabs_(p.y));
-  r.see(fabs_(p.z));
-  if (r.ok()) {
-    const float rw = rcp_ranged(p.w);
-    return mk3(div_shared(p.x, p.w, rw), div_shared(p.y, p.w, rw), div_shared(p.z, p.w, rw));
-  }
-  return mk3(p.x / p.w, p.y / p.w, p.z / p.w);
+  return perspective(mul44(inv_vp, mk4(uv.x * 2.0f - 1.0f, uv.y * 2.0f - 1.0f, depth, 1.0f)));
 }
 
 // SampleLevel(sampler_linear_clamp, uv, 0) restated with exact binary32 weights:
