@@ -689,6 +689,50 @@ __device__ __forceinline__ void spec_st(SpecPlanes p, size_t i, const SpecSample
 template <class Geo, int FORM>
 struct SpecTemporalF {
   static constexpr int kMinBlocks = 4;  // 64 registers (measured 15% faster)
+  // Balance-heuristic merge of the new sample with the previous reservoir (M > 0) over an
+  // arithmetic policy; false where that was left. 1920x1080: 90 -> 84 us from the surface
+  // planes, 97 -> 80 us from the raw G-buffer.
+  struct Merge {
+    bool use_prev;
+    float W, tf;
+  };
+  template <class A>
+  static __device__ __forceinline__ bool merge(const vlt_frame_params& fp, f3 pos, f3 n, float rough, f3 f0, f3 pn, float prough, f3 pf0, f3 nhp, f3 nrad, f3 rhp, f3 rrad, float rtf, uint32_t M, float W, uint32_t rng, Merge& out) {
+  A ar;
+  SpecTarget<A> cur;
+  cur.init(ar, vpos3(fp.view_pos), pos, n, rough, f0);
+  float sp_new, new_tf, new_w;
+  cur.eval(ar, nhp, nrad, &sp_new, &new_tf, &new_w);
+  float prev_w = W * (rtf * (float)M);
+  if (M > 0) {
+    SpecTarget<A> prv;
+    prv.init(ar, vpos3(fp.prev_view_pos), pos, pn, prough, pf0);
+    float ptoc = prv.tf(ar, nhp, nrad);
+    const float b_c = new_tf + ptoc * (float)M;
+    ar.see_unless(new_tf == 0.0f, new_tf);
+    ar.see_unless(new_tf == 0.0f, b_c);
+    float curr_m = A::div(new_tf, b_c);
+    if (new_tf == 0.0f) curr_m = 0.0f;
+    new_w = curr_m * new_w;
+    float ctop = cur.tf(ar, rhp, rrad);
+    float m_num = rtf * (float)M;
+    const float b_p = m_num + ctop;
+    ar.see_unless(m_num == 0.0f, m_num);
+    ar.see_unless(m_num == 0.0f, b_p);
+    float prev_m = A::div(m_num, b_p);
+    if (m_num == 0.0f) prev_m = 0.0f;
+    prev_w = prev_m * (ctop * W);
+    rtf = ctop;
+  }
+  float w_sum = prev_w + new_w;
+  ar.see_unless(w_sum == 0.0f, w_sum);
+  out.use_prev = ar.select(rng, prev_w, w_sum);
+  out.tf = out.use_prev ? rtf : new_tf;
+  ar.see_unless(!(out.tf > 0.0f), out.tf);
+  // a zero sum divided by a positive number is that zero
+  out.W = out.tf > 0.0f ? (w_sum == 0.0f ? w_sum : A::div(w_sum, out.tf)) : 0.0f;
+  return ar.ok();
+  }
   static __device__ __forceinline__ void run(int x0, int y0, vlt_frame_params fp, int w, int h, uint32_t m_cap, Geo geo, Geo prev_geo, const float* __restrict__ prev_depth, typename SpecStore<FORM>::CPtr prev, const float4* __restrict__ new_hp, const uint32_t* __restrict__ new_rad, typename SpecStore<FORM>::Ptr out, uint32_t frame_rand, uint32_t has_prev_frame) {
   int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
   if (!inb(x, y, w, h)) return;
@@ -743,42 +787,22 @@ struct SpecTemporalF {
   float rough = geo.rough(i);
   uint32_t mmax = f2u_rz((float)m_cap * rough);
   M = M < mmax ? M : mmax;
-  Ieee ar;
-  SpecTarget<Ieee> cur;
-  cur.init(ar, vpos3(fp.view_pos), pos, geo.normal(i), rough, geo.f0(i));
-  float sp_new, new_tf, new_w;
-  cur.eval(ar, nhp, nrad, &sp_new, &new_tf, &new_w);
-  float prev_w = W * (rtf * (float)M);
-  if (M > 0) {
-    SpecTarget<Ieee> prv;
-    prv.init(ar, vpos3(fp.prev_view_pos), pos, pn, prough, pf0);
-    float ptoc = prv.tf(ar, nhp, nrad);
-    float curr_m = new_tf / (new_tf + ptoc * (float)M);
-    if (new_tf == 0.0f) curr_m = 0.0f;
-    new_w = curr_m * new_w;
-    float ctop = cur.tf(ar, rhp, rrad);
-    float m_num = rtf * (float)M;
-    float prev_m = m_num / (m_num + ctop);
-    if (m_num == 0.0f) prev_m = 0.0f;
-    prev_w = prev_m * (ctop * W);
-    rtf = ctop;
-  }
+  const f3 n = geo.normal(i), f0 = geo.f0(i);
   uint32_t rng = lcg_init_with_seed((uint32_t)x, (uint32_t)y, frame_rand);
-  float w_sum = prev_w + new_w;
-  const bool use_prev = lcg_select(rng, prev_w, w_sum);
-  if (!use_prev) {
+  Merge m;
+  if (!merge<Ranged>(fp, pos, n, rough, f0, pn, prough, pf0, nhp, nrad, rhp, rrad, rtf, M, W, rng, m))
+    merge<Ieee>(fp, pos, n, rough, f0, pn, prough, pf0, nhp, nrad, rhp, rrad, rtf, M, W, rng, m);
+  if (!m.use_prev) {
     rhp = nhp;
     rrad_bits = nrad_bits;
     rrad = nrad;
-    rtf = new_tf;
   }
   M += 1;
-  W = rtf > 0.0f ? w_sum / rtf : 0.0f;
   SpecSample o;
   o.M = M;
-  o.W = W;
+  o.W = m.W;
   o.hit = rhp;
-  o.tf = rtf;
+  o.tf = m.tf;
   o.rad = rrad;
   o.rad_bits = rrad_bits;
   spec_st(out, i, o);
