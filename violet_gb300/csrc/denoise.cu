@@ -338,34 +338,62 @@ __device__ __forceinline__ f3 ycocg_to_rgb(f3 c) {
   return mk3(tmp + c.y, c.x + c.z, tmp - c.y);
 }
 
-// relax_fast_history_clamp.hlsl:11-75 (in place on the slow colour).
+// relax_fast_history_clamp.hlsl:11-75 (in place on the slow colour). A block decodes its
+// tile and a pixel around it into YCoCg once (each pixel decoded its nine neighbours: 18
+// R11G11B10 words); the twelve means share the reciprocal of 9: they are multiples of
+// 2^-48 within 2^36, and a special code makes the clamp's bounds NaN either way.
+// 1365x767: 45 -> 30 us, 1280x720 reference frame with the clamp 595 -> 579 us.
 struct DnFastClampF {
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, const uint2* __restrict__ fast, uint2* __restrict__ color) {
-  int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
+  struct Px {
+    float2 y, co, cg;  // diffuse, specular
+  };
+  __shared__ Px tile[(64 + 2) * (4 + 2)];  // the largest of the tile shapes, 64x4
+  const int bx = (int)blockDim.x, by = (int)blockDim.y, pw = bx + 2;
+  const int tid = (int)threadIdx.y * bx + (int)threadIdx.x;
+  __syncthreads();  // a persistent block's previous tile is done with the stage
+  for (int k = tid; k < pw * (by + 2); k += bx * by) {
+    const int r = k / pw;
+    int cx = x0 + k - r * pw - 1, cy = y0 + r - 1;
+    cx = cx < 0 ? 0 : (cx > w - 1 ? w - 1 : cx);
+    cy = cy < 0 ? 0 : (cy > h - 1 ? h - 1 : cy);
+    const uint2 f = fast[(size_t)cy * w + cx];
+    const f3 d = rgb_to_ycocg(col_diff(f)), s = rgb_to_ycocg(col_spec(f));
+    tile[k].y = make_float2(d.x, s.x);
+    tile[k].co = make_float2(d.y, s.y);
+    tile[k].cg = make_float2(d.z, s.z);
+  }
+  __syncthreads();
+  const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
   if (!inb(x, y, w, h)) return;
   size_t i = (size_t)y * w + x;
   f3 dm1 = mk3(0.0f), dm2 = mk3(0.0f), sm1 = mk3(0.0f), sm2 = mk3(0.0f);
-  for (int oy = -1; oy <= 1; ++oy) {
-    for (int ox = -1; ox <= 1; ++ox) {
-      int cx = x + ox, cy = y + oy;
-      cx = cx < 0 ? 0 : (cx > w - 1 ? w - 1 : cx);
-      cy = cy < 0 ? 0 : (cy > h - 1 ? h - 1 : cy);
-      uint2 f = fast[(size_t)cy * w + cx];
-      f3 d = rgb_to_ycocg(col_diff(f));
-      f3 s = rgb_to_ycocg(col_spec(f));
+#pragma unroll
+  for (int oy = 0; oy <= 2; ++oy) {
+#pragma unroll
+    for (int ox = 0; ox <= 2; ++ox) {
+      const Px t = tile[((int)threadIdx.y + oy) * pw + (int)threadIdx.x + ox];
+      const f3 d = mk3(t.y.x, t.co.x, t.cg.x), s = mk3(t.y.y, t.co.y, t.cg.y);
       dm1 = dm1 + d;
       dm2 = dm2 + d * d;
       sm1 = sm1 + s;
       sm2 = sm2 + s * s;
     }
   }
-  const float wsum = 9.0f;
-  dm1 = dm1 / wsum;
-  dm2 = dm2 / wsum;
-  sm1 = sm1 / wsum;
-  sm2 = sm2 / wsum;
-  f3 ddev = sqrt3(dm2 - dm1 * dm1) * 0.75f;
-  f3 sdev = sqrt3(sm2 - sm1 * sm1) * 0.75f;
+  const auto mean = [](f3 v) {
+    const float r = 1.0f / 9.0f;
+    return mk3(div_shared(v.x, 9.0f, r), div_shared(v.y, 9.0f, r), div_shared(v.z, 9.0f, r));
+  };
+  const auto root = [](f3 v) {
+    return mk3(v.x == 0.0f ? 0.0f : sqrt_ranged(v.x), v.y == 0.0f ? 0.0f : sqrt_ranged(v.y),
+               v.z == 0.0f ? 0.0f : sqrt_ranged(v.z));
+  };
+  dm1 = mean(dm1);
+  dm2 = mean(dm2);
+  sm1 = mean(sm1);
+  sm2 = mean(sm2);
+  f3 ddev = root(dm2 - dm1 * dm1) * 0.75f;
+  f3 sdev = root(sm2 - sm1 * sm1) * 0.75f;
   uint2 c = color[i];
   f3 d = rgb_to_ycocg(col_diff(c));
   f3 s = rgb_to_ycocg(col_spec(c));
