@@ -35,6 +35,7 @@ struct Object {
   float cam0[3];                      // camera position at frame 0
   float right[3], down[3], fwd[3];    // camera basis (world)
   float move[3];                      // per-frame translation direction
+  float top;                          // no heightfield value is above it, none below -top
 };
 
 VLT_HD uint64_t splitmix64(uint64_t x) {
@@ -85,6 +86,10 @@ VLT_HD Object make_object(uint64_t seed) {
     o.kz[k] = freq * sin_(ang);
     o.ph[k] = VLT_SCENE_TWO_PI * r.next();
   }
+  // The amplitudes added in height()'s order. |sin_| <= 1 (cos_poly adds a product that is
+  // not positive to 1) and rounding is monotonic, so no partial sum exceeds this one's.
+  o.top = 0.0f;
+  for (int k = 0; k < 4; ++k) o.top = o.top + o.amp[k];
   for (int s = 0; s < 4; ++s) {
     float rad = 0.5f + 1.0f * r.next();
     float cx = -4.0f + 8.0f * r.next();
@@ -165,29 +170,10 @@ struct Hit {
 
 #define VLT_SCENE_MAX_DIST 50.0f
 
-VLT_HD Hit trace(const Object& o, f3 org, f3 dir) {
-  Hit h;
-  h.t = 1e30f;
-  h.obj = -1;
-  // Ground: march t_i = 50 (i/64)^1.5, then bisect the first sign change.
-  float tprev = 0.0f;
-  for (int i = 1; i <= 64; ++i) {
-    float s = (float)i / 64.0f;
-    float t = VLT_SCENE_MAX_DIST * (s * sqrt_(s));
-    f3 p = org + t * dir;
-    if (p.y - height(o, p.x, p.z) < 0.0f) {
-      float lo = tprev, hi = t;
-      for (int b = 0; b < 16; ++b) {
-        float mid = 0.5f * (lo + hi);
-        f3 q = org + mid * dir;
-        if (q.y - height(o, q.x, q.z) < 0.0f) hi = mid; else lo = mid;
-      }
-      h.t = hi;
-      h.obj = 0;
-      break;
-    }
-    tprev = t;
-  }
+// The nearest sphere along the ray beyond 5 cm: its t and 1 + its index, or 1e30 and -1.
+VLT_HD void trace_spheres(const Object& o, f3 org, f3 dir, float* t_out, int* obj) {
+  *t_out = 1e30f;
+  *obj = -1;
   for (int s = 0; s < 4; ++s) {
     f3 c = mk3(o.sc[s][0], o.sc[s][1], o.sc[s][2]);
     float r = o.sc[s][3];
@@ -197,11 +183,90 @@ VLT_HD Hit trace(const Object& o, f3 org, f3 dir) {
     float disc = b * b - cc;
     if (disc > 0.0f) {
       float t = -b - sqrt_(disc);
-      if (t > 0.05f && t < h.t) {
-        h.t = t;
-        h.obj = 1 + s;
+      if (t > 0.05f && t < *t_out) {
+        *t_out = t;
+        *obj = 1 + s;
       }
     }
+  }
+}
+
+// Ground: march t_i = 50 (i/64)^1.5 to the first point below the heightfield, then bisect
+// the sign change 16 times; whether there is one, and its *hit with kBisect. A march that
+// has passed t_end ends: a crossing found later lies beyond it.
+//
+// The four sines of a sample are what a march costs, so a sample whose sign is already
+// certain is not evaluated; the answers are those of the march over all 64.
+// - At or above `top` no point is below the ground, and a ray that does not descend
+//   stays there (p.y is monotonic in t): it ends.
+// - Along the ray the heightfield rises by at most g = sum amp |kx dx + kz dz| per t, so a
+//   clearance c at t lasts until t + c / (g - dy), or for ever if dy >= g. The rounding of
+//   two samples is below 4e-3 in clearance for coordinates up to 1,024 (1.3e-4 per
+//   coordinate of p, 6e-4 for the sines' arguments, doubled, and 7e-4 for g's own
+//   cancellation over 50 m); 1e-2 is kept back, and beyond 1,024 every sample is evaluated.
+// A turn of the loop evaluates one sample of the march or of the bisection, whichever the
+// lane is at, so a warp takes as many turns as its slowest ray needs samples (with the
+// march and the bisection one after the other: 7 % more). A traced frame's rays from
+// 961 x 541 pixels, diffuse and specular: 749 us with every sample, 225 us so; what is
+// left is the instructions of the evaluated samples.
+template <bool kBisect>
+VLT_HD bool trace_ground(const Object& o, f3 org, f3 dir, float t_end, float* hit) {
+  float g = 0.0f;
+  for (int k = 0; k < 4; ++k) g = g + o.amp[k] * fabs_(o.kx[k] * dir.x + o.kz[k] * dir.z);
+  const float fall = g * 1.001f - dir.y;
+  const float far_x = fabs_(org.x) + VLT_SCENE_MAX_DIST * fabs_(dir.x);
+  const float far_y = fabs_(org.y) + VLT_SCENE_MAX_DIST * fabs_(dir.y);
+  const float far_z = fabs_(org.z) + VLT_SCENE_MAX_DIST * fabs_(dir.z);
+  const bool near = far_x <= 1024.0f && far_y <= 1024.0f && far_z <= 1024.0f;
+  int i = 0;           // the march's sample
+  int halvings = -1;   // of the bisection, -1 while marching
+  float clear = 0.0f;  // no sample up to here is below the ground
+  float lo = 0.0f, hi = 0.0f;
+  while (true) {
+    float t;
+    f3 p;
+    if (halvings < 0) {
+      do {
+        lo = hi;
+        if (lo > t_end || i == 64) return false;
+        ++i;
+        const float s = (float)i / 64.0f;
+        hi = VLT_SCENE_MAX_DIST * (s * sqrt_ranged(s));
+        p = org + hi * dir;
+        if (p.y >= o.top && dir.y >= 0.0f) return false;
+      } while (hi <= clear || p.y >= o.top);
+      t = hi;
+    } else {
+      t = 0.5f * (lo + hi);
+      p = org + t * dir;
+    }
+    const float c = p.y - height(o, p.x, p.z);
+    if (halvings < 0) {
+      if (c < 0.0f) {
+        if (!kBisect) return true;
+        halvings = 0;
+      } else if (near && c > 1e-2f) {
+        if (fall <= 0.0f) return false;
+        clear = t + (c - 1e-2f) / fall;
+      }
+    } else {
+      if (c < 0.0f) hi = t;
+      else lo = t;
+      if (++halvings == 16) {
+        *hit = hi;
+        return true;
+      }
+    }
+  }
+}
+
+VLT_HD Hit trace(const Object& o, f3 org, f3 dir) {
+  Hit h;
+  trace_spheres(o, org, dir, &h.t, &h.obj);
+  float t;
+  if (trace_ground<true>(o, org, dir, h.t, &t) && !(h.t < t)) {
+    h.t = t;
+    h.obj = 0;
   }
   if (h.obj < 0 || h.t > VLT_SCENE_MAX_DIST) {
     h.obj = -1;
@@ -215,6 +280,16 @@ VLT_HD Hit trace(const Object& o, f3 org, f3 dir) {
     h.n = normalize3(h.p - mk3(o.sc[s][0], o.sc[s][1], o.sc[s][2]));
   }
   return h;
+}
+
+// Whether trace() hits anything: the crossing alone decides for the ground, which the
+// march reaches within VLT_SCENE_MAX_DIST.
+VLT_HD bool occluded(const Object& o, f3 org, f3 dir) {
+  float t;
+  int obj;
+  trace_spheres(o, org, dir, &t, &obj);
+  if (obj > 0 && t <= VLT_SCENE_MAX_DIST) return true;
+  return trace_ground<false>(o, org, dir, 1e30f, &t);
 }
 
 // Quaternion helpers of brdf.hlsl / sampling.hlsl (get_rotation_to_z_from,
@@ -419,10 +494,10 @@ VLT_HD void trace_hit(const Object& o, uint64_t seed, f3 sun, const float* ray, 
   f3 color;
   float metallic, rough;
   material(seed, h.obj, h.p, &color, &metallic, &rough);
-  Hit sh = trace(o, h.p + 0.01f * h.n, sun);
+  const bool sun_visible = !occluded(o, h.p + 0.01f * h.n, sun);
   out[0] = h.p.x, out[1] = h.p.y, out[2] = h.p.z;
   out[4] = h.n.x, out[5] = h.n.y, out[6] = h.n.z;
-  out[7] = as_float(sh.obj < 0 ? 1u : 0u);  // sun visible
+  out[7] = as_float(sun_visible ? 1u : 0u);
   out[8] = h.n.x, out[9] = h.n.y, out[10] = h.n.z;
   out[11] = metallic;
   out[12] = color.x, out[13] = color.y, out[14] = color.z;
