@@ -411,7 +411,7 @@ __device__ __forceinline__ DiffSample load_diff(const uint4* p, size_t i, f3 pix
   s.W = rsv_decode_W(r.x);
   s.pos = hpn_pos(r.y, r.z);
   s.nrm = hpn_normal(r.z);
-  s.rad = unpack_r11g11b10(r.w);
+  s.rad = unpack_r11g11b10_int(r.w);
   diff_target(s, pix_pos, pix_n, dir, l2);
   return s;
 }
