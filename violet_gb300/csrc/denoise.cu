@@ -654,7 +654,9 @@ __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* 
       mk3(div_shared(r.y, ws.y, rw.y), div_shared(g.y, ws.y, rw.y), div_shared(b.y, ws.y, rw.y)));
   const size_t i = (size_t)y * w + x;
   if (o.color) o.color[i] = make_uint2(pd, ps);
-  if (o.var) o.var[i] = pack_half2(mk2(div_ranged(v.x, w2.x), div_ranged(v.y, w2.y)));
+  // a variance of -0 beside no tap keeps its sign
+  if (o.var)
+    o.var[i] = pack_half2(mk2(v.x > 0.0f ? div_ranged(v.x, w2.x) : v.x, v.y > 0.0f ? div_ranged(v.y, w2.y) : v.y));
   if (o.diff) o.diff[i] = pd;
   if (o.spec) o.spec[i] = ps;
 }
