@@ -544,7 +544,9 @@ struct DnAtrousF {
 // negative or not finite. Then no weight exponent is positive or NaN, and quotients
 // may be formed with a shared reciprocal (div_shared). Other blocks run the per-pixel
 // form. The per-pixel roots and quotients are the branch-free ones too (three iterations
-// at 1080p 379 -> 365 us against the IEEE operations).
+// at 1080p 379 -> 365 us against the IEEE operations). The normal weight's seven squarings
+// run for two taps of a row as a pair (reference-form frame at 1280x720 549 -> 544 us; in
+// the float forms, which wait for loads, it gained nothing).
 //
 // Bound by binary32 arithmetic: 1,834 warp instructions per 32 pixels (3,770 in the
 // per-pixel form) at 60 % issue, FMA pipe 49 % (the paired instructions take two of its
@@ -604,46 +606,60 @@ __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* 
     if (oy == 0) continue;
     if (CHECK && !inb(0, y + oy * step, 1, h)) continue;
 #pragma unroll
-    for (int ox = -2; ox <= 2; ++ox) {
-      if (ox == 0) continue;
-      if (CHECK && !inb(x + ox * step, 0, w, 1)) continue;
-      const int ax = ox < 0 ? -ox : ox, ay = oy < 0 ? -oy : oy, cls = ax + ay - 2;
-      const int j = li + oy * pw + ox * step;
-      const float4 ta = s[j].a, tb = s[j].b, tc = s[j].c;
-      const float2 tv = sv[j];
-      const float q = div_shared(fabsf(tc.w - cc.w), den[cls], rden[cls]);
-      const float2 nxy = __fmul2_rn(make_float2(cc.x, cc.y), make_float2(tc.x, tc.y));
-      float wn = __saturatef(nxy.x + nxy.y + cc.z * tc.z);
-      wn = pow_2k(wn, 7);
-      // exponent -(|dl| rcp_l + q): every term is finite and non-negative
-      const float2 dl = __fmul2_rn(__fadd2_rn(make_float2(tb.z, tb.w), neg_lum), rcp_l);
-      float2 e = __ffma2_rn(make_float2(fabsf(dl.x), fabsf(dl.y)), bc2(one), bc2(q));
-      e = __fmul2_rn(e, bc2(-VLT_LOG2E));
-      // exp2_select<false> for arguments <= 0: below -151 the clamp itself gives 0
-      e = make_float2(fmax_(e.x, -151.0f), fmax_(e.y, -151.0f));
-      const float2 t = __fadd2_rn(e, bc2(M));
-      const float2 f = __fadd2_rn(e, __ffma2_rn(t, bc2(-1.0f), bc2(M)));
-      float2 p = madd2(bc2(VLT_EXP2_C6), f, bc2(VLT_EXP2_C5), one);
-      p = madd2(p, f, bc2(VLT_EXP2_C4), one);
-      p = madd2(p, f, bc2(VLT_EXP2_C3), one);
-      p = madd2(p, f, bc2(VLT_EXP2_C2), one);
-      p = madd2(p, f, bc2(VLT_EXP2_C1), one);
-      p = madd2(p, f, bc2(VLT_EXP2_C0), one);
-      // 2^n as 2^e1 2^e2, e1 = max(n, -126): the integers sit in the shifted sums' low bits
-      const int tx = (int)as_uint(t.x), ty = (int)as_uint(t.y);
-      const int lo = 0x4B400000 - 126;
-      const int ex = tx < lo ? lo : tx, ey = ty < lo ? lo : ty;
-      const float2 s1 = make_float2(as_float(((uint32_t)ex << 23) + 0x3F800000u),
-                                    as_float(((uint32_t)ey << 23) + 0x3F800000u));
-      const float2 s2 = make_float2(as_float(((uint32_t)(tx - ex) << 23) + 0x3F800000u),
-                                    as_float(((uint32_t)(ty - ey) << 23) + 0x3F800000u));
-      p = __fmul2_rn(__fmul2_rn(p, s1), s2);
-      const float2 wt = __fmul2_rn(bc2(kw[ay] * kw[ax]), __fmul2_rn(bc2(wn), p));
-      r = madd2(wt, make_float2(ta.x, ta.y), r, one);
-      g = madd2(wt, make_float2(ta.z, ta.w), g, one);
-      b = madd2(wt, make_float2(tb.x, tb.y), b, one);
-      v = madd2(__fmul2_rn(wt, wt), tv, v, one);
-      ws = __ffma2_rn(wt, bc2(one), ws);
+    for (int side = -1; side <= 1; side += 2) {
+      const int j1 = li + oy * pw + side * step, j2 = j1 + side * step;
+      const bool in1 = !CHECK || inb(x + side * step, 0, w, 1), in2 = !CHECK || inb(x + 2 * side * step, 0, w, 1);
+      const auto cosine = [&](int j) {
+        const float4 tc = s[j].c;
+        const float2 nxy = __fmul2_rn(make_float2(cc.x, cc.y), make_float2(tc.x, tc.y));
+        return __saturatef(nxy.x + nxy.y + cc.z * tc.z);
+      };
+      const auto tap = [&](int j, int ax, float wn) {
+        const int ay = oy < 0 ? -oy : oy, cls = ax + ay - 2;
+        const float4 ta = s[j].a, tb = s[j].b, tc = s[j].c;
+        const float2 tv = sv[j];
+        const float q = div_shared(fabsf(tc.w - cc.w), den[cls], rden[cls]);
+        // exponent -(|dl| rcp_l + q): every term is finite and non-negative
+        const float2 dl = __fmul2_rn(__fadd2_rn(make_float2(tb.z, tb.w), neg_lum), rcp_l);
+        float2 e = __ffma2_rn(make_float2(fabsf(dl.x), fabsf(dl.y)), bc2(one), bc2(q));
+        e = __fmul2_rn(e, bc2(-VLT_LOG2E));
+        // exp2_select<false> for arguments <= 0: below -151 the clamp itself gives 0
+        e = make_float2(fmax_(e.x, -151.0f), fmax_(e.y, -151.0f));
+        const float2 t = __fadd2_rn(e, bc2(M));
+        const float2 f = __fadd2_rn(e, __ffma2_rn(t, bc2(-1.0f), bc2(M)));
+        float2 p = madd2(bc2(VLT_EXP2_C6), f, bc2(VLT_EXP2_C5), one);
+        p = madd2(p, f, bc2(VLT_EXP2_C4), one);
+        p = madd2(p, f, bc2(VLT_EXP2_C3), one);
+        p = madd2(p, f, bc2(VLT_EXP2_C2), one);
+        p = madd2(p, f, bc2(VLT_EXP2_C1), one);
+        p = madd2(p, f, bc2(VLT_EXP2_C0), one);
+        // 2^n as 2^e1 2^e2, e1 = max(n, -126): the integers sit in the shifted sums' low bits
+        const int tx = (int)as_uint(t.x), ty = (int)as_uint(t.y);
+        const int lo = 0x4B400000 - 126;
+        const int ex = tx < lo ? lo : tx, ey = ty < lo ? lo : ty;
+        const float2 s1 = make_float2(as_float(((uint32_t)ex << 23) + 0x3F800000u),
+                                      as_float(((uint32_t)ey << 23) + 0x3F800000u));
+        const float2 s2 = make_float2(as_float(((uint32_t)(tx - ex) << 23) + 0x3F800000u),
+                                      as_float(((uint32_t)(ty - ey) << 23) + 0x3F800000u));
+        p = __fmul2_rn(__fmul2_rn(p, s1), s2);
+        const float2 wt = __fmul2_rn(bc2(kw[ay] * kw[ax]), __fmul2_rn(bc2(wn), p));
+        r = madd2(wt, make_float2(ta.x, ta.y), r, one);
+        g = madd2(wt, make_float2(ta.z, ta.w), g, one);
+        b = madd2(wt, make_float2(tb.x, tb.y), b, one);
+        v = madd2(__fmul2_rn(wt, wt), tv, v, one);
+        ws = __ffma2_rn(wt, bc2(one), ws);
+      };
+      // The two taps' powers as a pair; the sums take the taps from left to right.
+      float2 nn = make_float2(in1 ? cosine(j1) : 0.0f, in2 ? cosine(j2) : 0.0f);
+#pragma unroll
+      for (int k = 0; k < 7; ++k) nn = __fmul2_rn(nn, nn);
+      if (side < 0) {
+        if (in2) tap(j2, 2, nn.y);
+        if (in1) tap(j1, 1, nn.x);
+      } else {
+        if (in1) tap(j1, 1, nn.x);
+        if (in2) tap(j2, 2, nn.y);
+      }
     }
   }
   // 1 <= ws <= 17; a sum too small for div_shared is stored as 0 either way

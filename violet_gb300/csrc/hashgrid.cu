@@ -346,7 +346,8 @@ struct HgSelResolveF {
 // of the list is unspecified). A block takes kCompactCells cells, each thread four at a
 // time, so that it issues all its loads at once and a grid of 2^22 cells takes 2,048
 // blocks: with one cell per thread the launch was 32,768 blocks of two barriers each, 25 us
-// for 16 MB that the L2 holds; the whole cache update at 2^22 cells and 921,600 queries 98.9 -> 79.0 us. V4: the selection is 16-byte aligned.
+// for 16 MB that the L2 holds; the whole cache update at 2^22 cells and 921,600 queries
+// 98.9 -> 79.0 us. V4: the selection is 16-byte aligned.
 constexpr uint32_t kCompactCells = 2048;
 template <bool V4>
 struct HgCompactF {
