@@ -105,15 +105,16 @@ FRAME_BYTES_PER_UPDATED_CELL = 37
 FORM = "f32"
 PASS_BYTES_PER_CELL = {"hg_decay": 2, "hg_compact": 4}
 # DRAM bytes per launch unit measured with ncu at 960x540, f32 (dram__bytes_read.sum +
-# dram__bytes_write.sum; the a-trous from one-pass counters, profiles/dn_atrous_f32_540p.md;
-# the specular spatial pass from its --set full capture, mean of its two launches,
+# dram__bytes_write.sum; the a-trous from its interleaved-record launches,
+# profiles/dn_atrous_f32_540p.md; the specular spatial pass the mean of its two launches,
 # profiles/spec_spatial_f32_540p.md).
-MEASURED_TRAFFIC_PER_UNIT = {"dn_atrous": 64.25, "spec_spatial": (36.013e6 + 0.507e6 + 34.377e6 + 0.322e6) / 2 / (960 * 540)}
-# Warp instructions per launch unit measured with ncu (smsp__inst_executed.sum of a
-# --set full capture / pixels, mean of two launches): the issue roofline of a pass
-# that is bound by instruction issue or latency rather than by HBM.
-MEASURED_WARP_INSTRUCTIONS_PER_UNIT = {"dn_atrous": (20.716e6 + 20.666e6) / 2 / (960 * 540),
-                                       "spec_spatial": (40.168e6 + 43.590e6) / 2 / (960 * 540)}
+MEASURED_TRAFFIC_PER_UNIT = {"dn_atrous": 64.1, "spec_spatial": (36.054e6 + 0.246e6 + 34.458e6 + 0.320e6) / 2 / (960 * 540)}
+# Warp instructions per launch unit measured with ncu (smsp__inst_executed.sum / pixels;
+# the a-trous the mean of its five launches, of which the first reads plain records): the
+# issue roofline of a pass that is bound by instruction issue or latency rather than by HBM.
+MEASURED_WARP_INSTRUCTIONS_PER_UNIT = {
+    "dn_atrous": (21.536e6 + 16.045e6 + 16.055e6 + 16.126e6 + 16.056e6) / 5 / (960 * 540),
+    "spec_spatial": (39.451e6 + 43.171e6) / 2 / (960 * 540)}
 ISSUE_SLOTS_PER_SM_CLOCK = 4  # one warp instruction per scheduler per clock, 4 schedulers per SM
 
 
