@@ -448,11 +448,19 @@ __device__ __forceinline__ void store_empty_diff(DiffF16Ptr out, size_t i) {
 // adaptive radius, plane-distance test, Jacobian clamped to [0, 1]).
 template <class Geo, int FORM>
 struct DiffSpatialF {
-  // 48 registers, 10 tiles per SM. Two 1080p passes: 298 us with the selected sample and its
-  // quotient test in registers at 64, 285 us carrying its pixel, 273 us at 48 (f32 frame
-  // 1,562 -> 1,537 us, 3840x2160 f16 6,038 -> 5,935 us, reference-form block at 1280x720 168.7
-  // -> 161.9 us). Issue-bound: 1,868 warp instructions per 32 pixels at 70 % issue.
+  // Reference and f16 form: 48 registers, 10 tiles of 128 threads per SM (3840x2160 f16 frame
+  // 6,038 -> 5,935 us, reference-form block at 1280x720 168.7 -> 161.9 us against 64). Bound by
+  // issue: 1,868 warp instructions per 32 pixels at 70 %.
+  // f32 form: its taps gather 48-byte records and are bound by the L1 where most of them are
+  // accepted (90 % of its throughput), so that more warps cost it the gathers' hits (51 % at
+  // 32 warps, 45 % at 40). Two passes in a frame of given candidates and in traced mode at
+  // 1920x1080, at 3840x2160 with the reference's knobs: 276, 384, 879 us at 48 registers and
+  // 40 warps; 288, 336, 762 at 64 and 32 with the selected sample in registers; 272, 335, 777 so:
+  // 56 registers and 6 tiles of 32x6 (32x4 tiles of as many warps share fewer of their
+  // taps: 272, 352, 801). Batches, whose views are small, keep 48.
   static constexpr int kMinBlocks = 5;
+  static constexpr int kTileX = 32, kTileY = FORM == FORM_F32 ? 6 : 4;
+  static constexpr int kTilesPerSM = FORM == FORM_F32 ? 6 : 0;
   static __device__ __forceinline__ void run(int x0, int y0, vlt_frame_params fp, int w, int h, DiffKnobs kn, Geo geo, const typename AoStore<FORM>::Filt* __restrict__ ao_tex, typename DiffStore<FORM>::CPtr in, typename DiffStore<FORM>::Ptr out, typename DiffStore<FORM>::Light* __restrict__ lighting, uint32_t frame_rand) {
   using S = DiffStore<FORM>;
   // The spiral's radius and angle offset of tap `it` depend only on it and the tap

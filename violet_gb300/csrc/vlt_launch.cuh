@@ -117,6 +117,23 @@ struct TileOf<F, decltype((void)F::kTileX)> {
   static constexpr int x = F::kTileX, y = F::kTileY;
 };
 
+// Register cap of a pass's single-view kernel as tiles of its own shape per SM
+// (F::kTilesPerSM), for caps between those of kMinBlocks; 0: kMinBlocks decides.
+template <class F, class = void>
+struct TilesPerSM {
+  static constexpr int value = 0;
+};
+template <class F>
+struct TilesPerSM<F, decltype((void)F::kTilesPerSM)> {
+  static constexpr int value = F::kTilesPerSM;
+};
+template <class F>
+struct GridBounds {
+  static constexpr bool own = TilesPerSM<F>::value > 0;
+  static constexpr int threads = own ? TileOf<F>::x * TileOf<F>::y : kMaxThreads;
+  static constexpr int blocks = own ? TilesPerSM<F>::value : MinBlocks<F>::value;
+};
+
 // Pixel rows per thread of a pass's tile (F::kRowsPerThread, default 1): a block of
 // bx x by threads covers a bx x (by * rows) tile.
 template <class F, class = void>
@@ -171,7 +188,7 @@ __device__ __forceinline__ void sort_rounds(SortedRounds& sr, const uint32_t key
 }
 
 template <class F, class... A>
-__global__ void __launch_bounds__(kMaxThreads, MinBlocks<F>::value) k_grid(A... a) {
+__global__ void __launch_bounds__(GridBounds<F>::threads, GridBounds<F>::blocks) k_grid(A... a) {
   F::run((int)(blockIdx.x * blockDim.x), (int)(blockIdx.y * blockDim.y * RowsOf<F>::value), a...);
 }
 
