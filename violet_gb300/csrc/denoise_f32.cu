@@ -218,7 +218,10 @@ struct Dn32TemporalF {
     return;
   }
   const float bw = (float)w, bh = (float)h;
-  f2 screen_uv = pixel_uv(x, y, w, h);
+  // Two IEEE divisions in the f32 form, the branch-free ones in the f16 form (3840x2160: 336
+  // against 345 us and 351 against 348 us for the pass).
+  const f2 screen_uv =
+      FORM == FORM_F32 ? mk2(((float)x + 0.5f) / bw, ((float)y + 0.5f) / bh) : pixel_uv(x, y, w, h);
   const f3 gnormal = geo.normal(i);
   const float grough = geo.rough(i);
   const float fwz = geo.fwz(i);
