@@ -1,5 +1,5 @@
-"""The query selection at the edges of the miss scatter's words, warps and blocks (64 queries
-per warp, 256 per block), on an empty grid, where every query is a miss, and on a filled one,
+"""The query selection at the edges of the miss scatter's words, warps and blocks (128 queries
+per warp, 512 per block), on an empty grid, where every query is a miss, and on a filled one,
 against the sequential loop. The scratch memory holds ones before the call: no bit of a
 query beyond the last may be read as a miss."""
 import ctypes as C
@@ -17,7 +17,7 @@ V = C.c_void_p
 
 
 @pytest.mark.parametrize("filled", [0, 12])
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 64, 65, 255, 256, 257, 1000, 4097])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 511, 512, 513, 1000, 4097])
 def test_select_at_scatter_edges(n, filled):
     import torch
 

@@ -243,13 +243,13 @@ struct HgSelAllocF {
 };
 
 // Scatter of the misses (the bits of miss_bits) into their buckets' segments. A thread takes
-// every 32nd of its warp's 32 * kScatter queries, so that its appends are in flight together
-// however many of the queries are misses: a first frame misses with all of them, a later
-// one with few. Whole selection at 921,600 queries and 2^22 cells, with 0 / 2 / 100 % of
-// the buckets' cells missing: one query per thread 37.4 / 45.5 / 86.7 us, two 34.4 / 42.1 /
-// 85.2, four 34.7 / 42.4 / 86.6; eight, walked bit by bit, 35 / - / 90, and at 57,600 queries
-// and 2^20 cells 33.4 where all are missing against 31.3.
-constexpr uint32_t kScatter = 2;
+// every 32nd of its warp's 32 * kScatter queries, each step for all of them before the next
+// one, so that its appends are in flight together however many of the queries are misses:
+// a first frame misses with all of them, a later one with few. This launch with none, the
+// queries of 5 % of the buckets and all queries missing: one query per thread 6.0 / 8.1 / 16.3
+// us at 1280x720 and 2^22 cells, 3.1 / 4.4 / 4.7 at 320x180 and 2^18; four 3.4 / 5.2 / 16.5 and
+// 3.1 / 4.7 / 4.8; eight, bit after bit, 2.8 / 6.9 / 18.1 and 3.0 / 6.0 / 9.2.
+constexpr uint32_t kScatter = 4;
 struct HgSelScatterF {
   static __device__ __forceinline__ void run(int x0, int y0, uint32_t max_q, const uint32_t* __restrict__ queries, const uint32_t* __restrict__ miss_bits, uint32_t* __restrict__ need_count, const uint32_t* __restrict__ need_offset, uint32_t* __restrict__ list) {
   const uint32_t lane = threadIdx.x & 31u, word = (((uint32_t)x0 + threadIdx.x) >> 5) * kScatter;
@@ -265,10 +265,13 @@ struct HgSelScatterF {
     bucket[k] = miss[k] ? queries[(size_t)((word + k) * 32u + lane) * Q_WORDS + Q_HASH] : 0u;
 #pragma unroll
   for (uint32_t k = 0; k < kScatter; ++k)
-    pos[k] = miss[k] ? need_offset[bucket[k]] + atomicAdd(need_count + bucket[k], 1u) : 0u;
+    pos[k] = miss[k] ? atomicAdd(need_count + bucket[k], 1u) : 0u;
 #pragma unroll
   for (uint32_t k = 0; k < kScatter; ++k)
-    if (miss[k]) list[pos[k]] = (word + k) * 32u + lane;
+    if (miss[k]) bucket[k] = need_offset[bucket[k]];
+#pragma unroll
+  for (uint32_t k = 0; k < kScatter; ++k)
+    if (miss[k]) list[bucket[k] + pos[k]] = (word + k) * 32u + lane;
 }
 };
 
