@@ -360,42 +360,33 @@ struct HgSelResolveF {
 
 // hash_grid_query_compact.hlsl:23-63 as the shader does it: a block appends its selected
 // cells through one global atomic (the blocks' order varies from run to run, and the order
-// of the list is unspecified). A block takes kCompactCells cells, each thread four at a
-// time, so that it issues all its loads at once and a grid of 2^22 cells takes 2,048
-// blocks: with one cell per thread the launch was 32,768 blocks of two barriers each, 25 us
-// for 16 MB that the L2 holds; the whole cache update at 2^22 cells and 921,600 queries
-// 98.9 -> 79.0 us. V4: the selection is 16-byte aligned.
-constexpr uint32_t kCompactCells = 2048;
-template <bool V4>
+// of the list is unspecified). A block takes kCompactCells cells, each warp a run of them
+// whose words its lanes load at once, 32 neighbours per load, and append in their order, so
+// that the loads coalesce and, however many cells are selected, the stores too. At 2^22 cells
+// with 0.1 / 10 / 100 % selected, in cache: 5.2 / 6.9 / 8.3 us, one cell per thread 18.8 / 24.1 /
+// 24.7 (32,768 blocks of two barriers), four neighbours per thread in 16-byte loads 5.1 / 7.2 /
+// 38.3 (scattered stores); at 4,096 cells 2.3 / 2.4 / 2.5, 2.2 / 2.3 / 2.3 and 2.6 / 2.7 / 4.3. Blocks of
+// 2,048 cells are slower on the small grids (3.0), of 512 on the large ones (6.6 / 9.1 / 9.9).
+constexpr uint32_t kCompactCells = 1024;
 struct HgCompactF {
   static __device__ __forceinline__ void run(int x0, int y0, uint32_t num_cells, uint32_t qmask, const uint32_t* __restrict__ selection, uint32_t* __restrict__ idx, uint32_t* __restrict__ addr, uint32_t* __restrict__ count) {
-  constexpr uint32_t kRounds = kCompactCells / (4 * kBlock1D);
-  __shared__ uint32_t warp_cnt[kBlock1D / 32], block_base;
+  constexpr uint32_t kWarps = kBlock1D / 32, kRounds = kCompactCells / kBlock1D;
+  __shared__ uint32_t warp_cnt[kWarps], block_base;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-  const uint32_t first = (uint32_t)x0 / kBlock1D * kCompactCells + 4 * threadIdx.x;
-  uint4 sel[kRounds];
-  uint32_t n = 0;
+  const uint32_t first = (uint32_t)x0 / kBlock1D * kCompactCells + wid * (32u * kRounds) + lane;
+  uint32_t sel[kRounds], n = 0;
 #pragma unroll
   for (uint32_t r = 0; r < kRounds; ++r) {
-    const uint32_t c = first + r * 4 * kBlock1D;  // num_cells is a multiple of 256
-    sel[r] = make_uint4(0u, 0u, 0u, 0u);
-    if (c < num_cells) {
-      if (V4) sel[r] = *(const uint4*)(selection + c);
-      else sel[r] = make_uint4(selection[c], selection[c + 1], selection[c + 2], selection[c + 3]);
-    }
-    n += (sel[r].x != 0u) + (sel[r].y != 0u) + (sel[r].z != 0u) + (sel[r].w != 0u);
+    const uint32_t c = first + r * 32u;
+    sel[r] = c < num_cells ? selection[c] : 0u;
   }
-  uint32_t incl = n;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= (uint32_t)d) incl += v;
-  }
-  if (lane == 31u) warp_cnt[wid] = incl;
+  for (uint32_t r = 0; r < kRounds; ++r) n += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, sel[r] != 0u));
+  if (lane == 0u) warp_cnt[wid] = n;
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t tot = 0;
-    for (uint32_t k = 0; k < kBlock1D / 32; ++k) {
+    for (uint32_t k = 0; k < kWarps; ++k) {
       const uint32_t v = warp_cnt[k];
       warp_cnt[k] = tot;
       tot += v;
@@ -403,17 +394,16 @@ struct HgCompactF {
     block_base = tot ? atomicAdd(count, tot) : 0u;
   }
   __syncthreads();
-  uint32_t pos = block_base + warp_cnt[wid] + incl - n;
+  uint32_t base = block_base + warp_cnt[wid];
 #pragma unroll
   for (uint32_t r = 0; r < kRounds; ++r) {
-    const uint32_t c = first + r * 4 * kBlock1D, v[4] = {sel[r].x, sel[r].y, sel[r].z, sel[r].w};
-#pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) {
-      if (v[k] == 0u) continue;
-      idx[pos] = v[k] & qmask;
-      addr[pos] = c + k;
-      ++pos;
+    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, sel[r] != 0u);
+    if (sel[r] != 0u) {
+      const uint32_t pos = base + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+      idx[pos] = sel[r] & qmask;
+      addr[pos] = first + r * 32u;
     }
+    base += (uint32_t)__popc(bal);
   }
   __syncthreads();  // the shared words are reused by the block's next chunk (persistent launches)
 }
@@ -574,10 +564,7 @@ void launch_hg_compact(const Exec& ex, const HashGridDims& d, const uint32_t* se
     uint32_t nc = d.num_cells();
     uint32_t qmask = (1u << d.query_bits()) - 1u;
     const uint32_t n = (nc + kCompactCells - 1) / kCompactCells * kBlock1D;  // one block per chunk
-    if (((uintptr_t)selection & 15u) == 0)
-      launch1d<HgCompactF<true>>(ex, "hg_compact", n, nc, qmask, selection, idx, addr, count);
-    else
-      launch1d<HgCompactF<false>>(ex, "hg_compact", n, nc, qmask, selection, idx, addr, count);
+    launch1d<HgCompactF>(ex, "hg_compact", n, nc, qmask, selection, idx, addr, count);
     return;
   }
   HgCompactSel::Args a = {selection, (1u << d.query_bits()) - 1u, idx, addr};
