@@ -636,14 +636,15 @@ __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* 
         p = madd2(p, f, bc2(VLT_EXP2_C2), one);
         p = madd2(p, f, bc2(VLT_EXP2_C1), one);
         p = madd2(p, f, bc2(VLT_EXP2_C0), one);
-        // 2^n as 2^e1 2^e2, e1 = max(n, -126): the integers sit in the shifted sums' low bits
+        // 2^n as 2^max(n, -126) 2^min(n + 126, 0): the integers sit in the shifted sums' low bits.
+        // (With the second exponent as n - max(n, -126) the compiled kernel takes it as 0.)
         const int tx = (int)as_uint(t.x), ty = (int)as_uint(t.y);
         const int lo = 0x4B400000 - 126;
-        const int ex = tx < lo ? lo : tx, ey = ty < lo ? lo : ty;
-        const float2 s1 = make_float2(as_float(((uint32_t)ex << 23) + 0x3F800000u),
-                                      as_float(((uint32_t)ey << 23) + 0x3F800000u));
-        const float2 s2 = make_float2(as_float(((uint32_t)(tx - ex) << 23) + 0x3F800000u),
-                                      as_float(((uint32_t)(ty - ey) << 23) + 0x3F800000u));
+        const uint32_t one2 = 0x3F800000u - ((uint32_t)lo << 23);
+        const float2 s1 = make_float2(as_float(((uint32_t)max(tx, lo) << 23) + 0x3F800000u),
+                                      as_float(((uint32_t)max(ty, lo) << 23) + 0x3F800000u));
+        const float2 s2 = make_float2(as_float(((uint32_t)min(tx, lo) << 23) + one2),
+                                      as_float(((uint32_t)min(ty, lo) << 23) + one2));
         p = __fmul2_rn(__fmul2_rn(p, s1), s2);
         const float2 wt = __fmul2_rn(bc2(kw[ay] * kw[ax]), __fmul2_rn(bc2(wn), p));
         r = madd2(wt, make_float2(ta.x, ta.y), r, one);
