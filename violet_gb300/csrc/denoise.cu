@@ -541,15 +541,22 @@ struct DnAtrousF {
 // pairs, and the paired binary32 instructions (one IEEE operation per component, the
 // same bits) halve the issue slots of the parts that run per channel.
 //
-// Two things the per-pixel form guards per tap are settled per block. A block is
-// `tame` when every staged colour and variance is finite, no variance is negative,
-// every depth is 0 or of a magnitude in [2^-70, 2^70] and no fwidth_z of the tile is
-// negative or not finite. Then no weight exponent is positive or NaN, and quotients
-// may be formed with a shared reciprocal (div_shared). Other blocks run the per-pixel
-// form. The per-pixel roots and quotients are the branch-free ones too (three iterations
-// at 1080p 379 -> 365 us against the IEEE operations). The normal weight's seven squarings
-// run for two taps of a row as a pair (reference-form frame at 1280x720 549 -> 544 us; in
-// the float forms, which wait for loads, it gained nothing).
+// What the per-pixel form guards per tap is settled per block. The geometry is `tame`
+// when every depth is 0 or of a magnitude in [2^-70, 2^70] and no fwidth_z of the tile is
+// negative or not finite. Then the depth terms' quotients may be formed with a shared
+// reciprocal (div_shared) and no weight exponent is positive; other blocks run the
+// per-pixel form. The values are `ordinary` when every staged colour and variance is
+// finite and no variance is negative. Then the per-pixel roots and quotients are the
+// branch-free ones (three iterations at 1080p 379 -> 365 us against the IEEE operations);
+// blocks with other values take those few operations as IEEE ones, and the rest of the
+// arithmetic is the same for infinities and NaN: an overflowed variance, which the
+// iterations spread over ever more blocks (0.9 % of them in the first, 31 % in the fifth
+// in a walk at 1080p), does not take a block off the tile. An iteration at 1080p over one
+// special variance per tile, steps 1 / 4 / 16: 337 / 201 / 195 us in the per-pixel form, 148 / 136 / 160
+// so; all variances infinite at step 16: 398 (328 in the per-pixel form alone) and 210.
+// The normal weight's seven squarings run for two taps of a row as a pair (reference-form
+// frame at 1280x720 549 -> 544 us; in the float forms, which wait for loads, it gained
+// nothing).
 //
 // Bound by binary32 arithmetic: 1,834 warp instructions per 32 pixels (3,770 in the
 // per-pixel form) at 60 % issue, FMA pipe 49 % (the paired instructions take two of its
@@ -585,19 +592,31 @@ struct AtrousOut {
   uint32_t* __restrict__ spec;
 };
 
-// One output pixel of a tame block; s is the staged tile, li the pixel's place in it,
-// pw the tile's row pitch. CHECK: the footprint may leave the image.
-template <bool CHECK>
+// max(a, b), NaN where a is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// One output pixel of a block of tame geometry; s is the staged tile, li the pixel's place
+// in it, pw the tile's row pitch. CHECK: the footprint may leave the image.
+template <bool CHECK, bool ORDINARY>
 __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* sv, int li, int pw, int x, int y,
                                                int w, int h, float fwz, float3 td, int step, const AtrousOut& o, float one) {
   const float4 ca = s[li].a, cb = s[li].b, cc = s[li].c;
   const float2 cv = sv[li];
   const float eps = 1e-8f;
   const float2 neg_lum = make_float2(-cb.z, -cb.w);
-  // A tame block's operands are in the branch-free forms' ranges: a variance is 0 or a
-  // half of at least 2^-24, the denominators lie in [1e-8, 1e8], the weight sum in [1, 17].
-  const float2 sd = make_float2(cv.x > 0.0f ? sqrt_ranged(cv.x) : 0.0f, cv.y > 0.0f ? sqrt_ranged(cv.y) : 0.0f);
-  const float2 rcp_l = make_float2(rcp_ranged(4.0f * sd.x + eps), rcp_ranged(4.0f * sd.y + eps));
+  // Ordinary operands are in the branch-free forms' ranges: a variance is 0 or a half of at
+  // least 2^-24, the denominators lie in [1e-8, 1e8], the weight sum in [1, 17].
+  float2 rcp_l;
+  if (ORDINARY) {
+    const float2 sd = make_float2(cv.x > 0.0f ? sqrt_ranged(cv.x) : 0.0f, cv.y > 0.0f ? sqrt_ranged(cv.y) : 0.0f);
+    rcp_l = make_float2(rcp_ranged(4.0f * sd.x + eps), rcp_ranged(4.0f * sd.y + eps));
+  } else {
+    rcp_l = make_float2(1.0f / (4.0f * sqrt_(cv.x) + eps), 1.0f / (4.0f * sqrt_(cv.y) + eps));
+  }
   const float den[3] = {fwz * td.x + eps, fwz * td.y + eps, fwz * td.z + eps};
   const float rden[3] = {rcp_ranged(den[0]), rcp_ranged(den[1]), rcp_ranged(den[2])};
   float2 r = make_float2(ca.x, ca.y), g = make_float2(ca.z, ca.w), b = make_float2(cb.x, cb.y), v = cv,
@@ -622,12 +641,13 @@ __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* 
         const float4 ta = s[j].a, tb = s[j].b, tc = s[j].c;
         const float2 tv = sv[j];
         const float q = div_shared(fabsf(tc.w - cc.w), den[cls], rden[cls]);
-        // exponent -(|dl| rcp_l + q): every term is finite and non-negative
+        // exponent -(|dl| rcp_l + q): every term is non-negative or NaN, q finite
         const float2 dl = __fmul2_rn(__fadd2_rn(make_float2(tb.z, tb.w), neg_lum), rcp_l);
         float2 e = __ffma2_rn(make_float2(fabsf(dl.x), fabsf(dl.y)), bc2(one), bc2(q));
         e = __fmul2_rn(e, bc2(-VLT_LOG2E));
-        // exp2_select<false> for arguments <= 0: below -151 the clamp itself gives 0
-        e = make_float2(fmax_(e.x, -151.0f), fmax_(e.y, -151.0f));
+        // exp2_select<false> for arguments <= 0 or NaN: below -151 the clamp itself gives 0
+        e = ORDINARY ? make_float2(fmax_(e.x, -151.0f), fmax_(e.y, -151.0f))
+                     : make_float2(max_nan(e.x, -151.0f), max_nan(e.y, -151.0f));
         const float2 t = __fadd2_rn(e, bc2(M));
         const float2 f = __fadd2_rn(e, __ffma2_rn(t, bc2(-1.0f), bc2(M)));
         float2 p = madd2(bc2(VLT_EXP2_C6), f, bc2(VLT_EXP2_C5), one);
@@ -666,17 +686,25 @@ __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* 
       }
     }
   }
-  // 1 <= ws <= 17; a sum too small for div_shared is stored as 0 either way
-  const float2 rw = make_float2(rcp_ranged(ws.x), rcp_ranged(ws.y)), w2 = __fmul2_rn(ws, ws);
-  const uint32_t pd = pack_r11g11b10(
-      mk3(div_shared(r.x, ws.x, rw.x), div_shared(g.x, ws.x, rw.x), div_shared(b.x, ws.x, rw.x)));
-  const uint32_t ps = pack_r11g11b10(
-      mk3(div_shared(r.y, ws.y, rw.y), div_shared(g.y, ws.y, rw.y), div_shared(b.y, ws.y, rw.y)));
+  const float2 w2 = __fmul2_rn(ws, ws);
+  f3 d, sp;
+  f2 vd;
+  if (ORDINARY) {
+    // 1 <= ws <= 17; a sum too small for div_shared is stored as 0 either way, and a variance
+    // of -0 beside no tap keeps its sign
+    const float2 rw = make_float2(rcp_ranged(ws.x), rcp_ranged(ws.y));
+    d = mk3(div_shared(r.x, ws.x, rw.x), div_shared(g.x, ws.x, rw.x), div_shared(b.x, ws.x, rw.x));
+    sp = mk3(div_shared(r.y, ws.y, rw.y), div_shared(g.y, ws.y, rw.y), div_shared(b.y, ws.y, rw.y));
+    vd = mk2(v.x > 0.0f ? div_ranged(v.x, w2.x) : v.x, v.y > 0.0f ? div_ranged(v.y, w2.y) : v.y);
+  } else {
+    d = mk3(r.x, g.x, b.x) / ws.x;
+    sp = mk3(r.y, g.y, b.y) / ws.y;
+    vd = mk2(v.x / w2.x, v.y / w2.y);
+  }
+  const uint32_t pd = pack_r11g11b10(d), ps = pack_r11g11b10(sp);
   const size_t i = (size_t)y * w + x;
   if (o.color) o.color[i] = make_uint2(pd, ps);
-  // a variance of -0 beside no tap keeps its sign
-  if (o.var)
-    o.var[i] = pack_half2(mk2(v.x > 0.0f ? div_ranged(v.x, w2.x) : v.x, v.y > 0.0f ? div_ranged(v.y, w2.y) : v.y));
+  if (o.var) o.var[i] = pack_half2(vd);
   if (o.diff) o.diff[i] = pd;
   if (o.spec) o.spec[i] = ps;
 }
@@ -698,7 +726,12 @@ __global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
   // Tile rows: blockIdx.y counts (group of 8 * step image rows, phase within it).
   const int group = (int)blockIdx.y / step, phase = (int)blockIdx.y - group * step;
   const int x0 = (int)blockIdx.x * kAtrousTileX, y0 = group * (kAtrousTileRows * step) + phase;
-  bool tame = true;
+  uint32_t odd = 0u;  // 1: a value, 2: the geometry
+  const auto tame_depth = [](float d) { return d == 0.0f || (fabsf(d) >= 0x1p-70f && fabsf(d) <= 0x1p70f); };
+  const auto tame_fwz = [](float f) { return f >= 0.0f && f < 1e6f; };
+  const auto in_tile = [=](int row, int col) {
+    return row >= 2 && row < kAtrousTileRows + 2 && col >= 2 * step && col < kAtrousTileX + 2 * step;
+  };
   for (int k = tid; k < np; k += NT) {
     const int row = (int)__umulhi((uint32_t)k, pitch_inv), col = k - row * pw;  // k / pw (host: exact for k < np)
     const int gx = x0 + col - 2 * step, gy = y0 + (row - 2) * step;
@@ -716,19 +749,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
     s[k] = px;
     const f2 v = unpack_half2(vw);
     sv[k] = make_float2(v.x, v.y);
-    const float ad = fabsf(dep);
-    // exponent code 31: an infinity or a NaN
-    const bool special = (cw.x & 0x7C0u) == 0x7C0u || (cw.x & 0x3E0000u) == 0x3E0000u ||
-                         (cw.x & 0xF8000000u) == 0xF8000000u || (cw.y & 0x7C0u) == 0x7C0u ||
-                         (cw.y & 0x3E0000u) == 0x3E0000u || (cw.y & 0xF8000000u) == 0xF8000000u;
-    tame = tame && !special && v.x >= 0.0f && v.y >= 0.0f && v.x < 1e6f && v.y < 1e6f &&
-           (dep == 0.0f || (ad >= 0x1p-70f && ad <= 0x1p70f));
-    if (row >= 2 && row < kAtrousTileRows + 2 && col >= 2 * step && col < kAtrousTileX + 2 * step) {
-      const float fz = geo.fwz(i);
-      tame = tame && fz >= 0.0f && fz < 1e6f;
-    }
+    // a luminance is finite where its channels are
+    if (!(px.b.z < 1e6f && px.b.w < 1e6f && v.x >= 0.0f && v.y >= 0.0f && v.x < 1e6f && v.y < 1e6f)) odd |= 1u;
+    if (!tame_depth(dep)) odd |= 2u;
+    if (in_tile(row, col) && !tame_fwz(geo.fwz(i))) odd |= 2u;
   }
-  tame = __syncthreads_and(tame);
+  const bool ordinary = __syncthreads_and(odd == 0u);
+  const bool tame = ordinary || __syncthreads_and(odd < 2u);
   const float3 td = make_float3(taps.dist[5], taps.dist[4], taps.dist[0]);
   const bool interior = x0 - 2 * step >= 0 && x0 + kAtrousTileX - 1 + 2 * step <= w - 1 && y0 - 2 * step >= 0 &&
                         y0 + (kAtrousTileRows + 1) * step <= h - 1;
@@ -743,8 +770,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
     }
     const float fwz = geo.fwz((size_t)y * w + x);
     const int li = (row + 2) * pw + tx + 2 * step;
-    if (interior) atrous_tile_px<false>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
-    else atrous_tile_px<true>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
+    if (!ordinary) atrous_tile_px<true, false>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
+    else if (interior) atrous_tile_px<false, true>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
+    else atrous_tile_px<true, true>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
   }
 }
 
