@@ -588,8 +588,9 @@ struct SpecTarget {
     r2 = roughness * roughness;
     const f3 d = view_pos - p;
     const float d2 = dot3(d, d);
-    ar.see(d2);
-    v = d * A::rsqrt(d2);
+    const float rd = A::rsqrt(d2);
+    ar.see_rsqrt(rd);
+    v = d * rd;
     nov = saturate(dot3(n, v));
     ar.see_unless(nov == 0.0f, nov);
     const float sq = A::sqrt((-r2 * nov + nov) * nov + r2);
@@ -614,8 +615,9 @@ struct SpecTarget {
   __device__ __forceinline__ void eval(A& ar, f3 hit, f3 rad, float* source_pdf, float* tf, float* w) const {
     const f3 dl = hit - pos;
     const float l2 = dot3(dl, dl);
-    ar.see(l2);
-    const f3 l = dl * A::rsqrt(l2);
+    const float rl = A::rsqrt(l2);
+    ar.see_rsqrt(rl);
+    const f3 l = dl * rl;
     const f3 dh = v + l;
     const float h2 = dot3(dh, dh);
     ar.see(h2);
@@ -944,12 +946,11 @@ __device__ __forceinline__ bool spec_spatial_px_as(int x, int y, const vlt_frame
     W = ctf > 0.0f ? (w_sum == 0.0f ? w_sum : A::div(w_sum, ctf)) : 0.0f;
   }
   const f3 dl = hit - pos;
-  const float l2 = dot3(dl, dl);
-  ar.see(l2);
-  const float ray_len = A::sqrt(l2);
+  const float ray_len = A::sqrt(dot3(dl, dl)), inv_len = A::rcp(ray_len);
+  ar.see_rsqrt(inv_len);
   f3 li = mk3(0.0f);
   if (lighting) {
-    const f3 l = dl * A::rcp(ray_len);
+    const f3 l = dl * inv_len;
     const f3 dh = center.v + l;
     const float h2 = dot3(dh, dh);
     ar.see(h2);
