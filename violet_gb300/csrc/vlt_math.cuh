@@ -133,18 +133,20 @@ VLT_HD float fma_(float a, float b, float c) {
 }
 
 // Correctly rounded division and square roots without branches, for operands of magnitude
-// in [2^-60, 2^60] (a dividend may also be 0; the sign of its zero quotient may then
-// differ from the IEEE one). An approximate reciprocal or root, one Newton step where the
+// in [2^-60, 2^60], roots of any finite number of at least 2^-100 (a dividend may also be 0;
+// the sign of its zero quotient may then differ from the IEEE one). An approximate reciprocal or root, one Newton step where the
 // result needs it, and one correction by the exact residual (Markstein 1990, "Computation
 // of elementary functions on the IBM RISC System/6000 processor"):
 //   reciprocal  r = r0 + r0 (1 - b r0)
 //   quotient    q = a r, then q + r (a - b q)
 //   root        g = x y, then g + (y / 2) (x - g g)
-// Exhaustive comparisons on the GPU found no difference from the IEEE operations: the
-// reciprocal and the root over every binary32 in [2^-100, 2^100], the quotient over all
-// 2^46 pairs of mantissas (the approximate reciprocal scales exactly over the exponents),
-// with this reciprocal and with the correctly rounded one. Without the Newton step 79,381
-// of the quotients differed. The host build uses the language's operations.
+// No difference from the IEEE operations: the reciprocal over every binary32 in [2^-100,
+// 2^100] and the roots over every one from 2^-100 up (tests/native/exact_math_check.cu, with
+// quotients of 2^32 random pairs and 3 * 2^30 next to the middle of two neighbours); the
+// quotient over all 2^46 pairs of mantissas (one run; the approximate reciprocal scales
+// exactly over the exponents), with this reciprocal and with the correctly rounded one.
+// Without the Newton step 79,381 of the quotients differed. The host build uses the
+// language's operations.
 VLT_HD float rcp_ranged(float b) {
 #if defined(__CUDA_ARCH__)
   float r;
