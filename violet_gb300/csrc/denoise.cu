@@ -270,6 +270,8 @@ __device__ __forceinline__ float quad_max_len(const uint8_t* __restrict__ len, i
 
 // --------------------------------------------------------- disocclusion fix
 
+namespace {
+
 // Sums of the short-history filters (the weight without luminance terms is the same for
 // both channels), and that weight.
 struct FilterSums {
@@ -289,6 +291,8 @@ __device__ __forceinline__ float short_weight(const ShortPixel& c, const Geo& ge
   const float wz = -fabs_(geo.dep(j) - c.depth) / (c.fz_sigma * tap_dist + 1e-8f);
   return pow_2k(saturate(dot3(c.normal, geo.normal(j))), sigma_n_log2) * exp_(wz);
 }
+
+}  // namespace
 
 // relax_disocclusion_fix.hlsl:27-122. Pixels without geometry (history 0) are not
 // written by the shader; here they get zeros.

@@ -401,6 +401,8 @@ struct Dn32TemporalF {
 
 // ----------------------------------------------------------- disocclusion fix
 
+namespace {
+
 // Sums of the short-history filters (the weight without luminance terms is the same for
 // both channels), and that weight.
 template <bool CENTERED>
@@ -428,6 +430,8 @@ __device__ __forceinline__ float short_weight(const ShortPixel& c, const Geo& ge
   const float n_dot = saturate(fma_(c.normal.z, n.z, fma_(c.normal.y, n.y, c.normal.x * n.x)));
   return pow_2k(n_dot, sigma_n_log2) * exp_fma(wz);
 }
+
+}  // namespace
 
 template <class Geo, int FORM>
 struct Dn32FixF {
