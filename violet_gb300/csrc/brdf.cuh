@@ -13,15 +13,6 @@ __device__ __forceinline__ float d_ggx(float noh, float roughness) {
   return k * k * VLT_ONE_OVER_PI;
 }
 
-// (smith_lambda + 1) * cos (ind_spec_temporal_resample.hlsl:48-53).
-__device__ __forceinline__ float lambda_pomc(float c, float roughness) {
-  float r2 = roughness * roughness;
-  return (c + sqrt_((-r2 * c + c) * c + r2)) / 2.0f;
-}
-
-// One factor of smith_G2_over_G1_height_correlated_GGX (brdf.hlsl:133-137).
-__device__ __forceinline__ float g_k(float c, float r2) { return sqrt_((-r2 * c + c) * c + r2) / c; }
-
 __device__ __forceinline__ f3 f_schlick(float u, f3 f0) {
   float f = pow5(1.0f - u);
   return mk3(f + f0.x * (1.0f - f), f + f0.y * (1.0f - f), f + f0.z * (1.0f - f));

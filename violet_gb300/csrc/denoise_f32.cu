@@ -631,7 +631,7 @@ __device__ __forceinline__ void store_rec(AtrousMid* __restrict__ p, size_t i, f
 }
 
 // What a pixel's weights need of it: the base-2 reciprocals of the luminance deviation and
-// of the depth terms by distance (weight_rz).
+// of the depth terms by tap distance, for (|ox|, |oy|) = (1,1), (1,2) or (2,1), and (2,2).
 struct AtrousCentre {
   float depth, r11, r12, r22;
   f3 normal;

@@ -594,10 +594,10 @@ struct SpecTarget {
     nov = saturate(dot3(n, v));
     ar.see_unless(nov == 0.0f, nov);
     const float sq = A::sqrt((-r2 * nov + nov) * nov + r2);
-    lp = (nov + sq) / 2.0f;   // lambda_pomc
-    kv = A::div(sq, nov);     // g_k
+    lp = (nov + sq) / 2.0f;  // (smith_lambda + 1) * cos (ind_spec_temporal_resample.hlsl:48-53)
+    kv = A::div(sq, nov);    // one factor of smith_G2_over_G1_height_correlated_GGX (brdf.hlsl:133-137)
   }
-  // (1 + kv) / (kv + g_k(nol)), 0 where either cosine is 0.
+  // (1 + kv) over the sum of kv and the same factor of nol, 0 where either cosine is 0.
   __device__ __forceinline__ float smith(A& ar, float nol) const {
     ar.see_unless(nol == 0.0f, nol);
     float g = A::div(1.0f + kv, kv + A::div(A::sqrt((-r2 * nol + nol) * nol + r2), nol));
