@@ -35,10 +35,6 @@ struct GraphEntry {
   uint64_t last_use = 0;
 };
 
-// Candidate launch shapes: five tile shapes, each one tile per block and persistent.
-const TileShape kCandidates[VLT_TILE_CANDIDATES] = {{32, 4, 0}, {16, 8, 0}, {32, 8, 0}, {16, 16, 0}, {64, 4, 0},
-                                                    {32, 4, 1}, {16, 8, 1}, {32, 8, 1}, {16, 16, 1}, {64, 4, 1}};
-
 struct TuneRec {
   std::string name;
   double ns[VLT_TILE_CANDIDATES] = {};
@@ -156,7 +152,7 @@ std::vector<Group> order_chunk(const std::vector<const Recorder*>& recs) {
 
 TileShape shape_for(vlt_batch* b, const Job& j) {
   if (!j.one_d) {
-    if (b->tune_left > 0) return kCandidates[b->tune_index % VLT_TILE_CANDIDATES];
+    if (b->tune_left > 0) return kTileCandidates[b->tune_index % VLT_TILE_CANDIDATES];
     auto it = b->shapes.find((const void*)j.prepare);
     if (it != b->shapes.end()) return it->second;
   }
@@ -180,7 +176,7 @@ void finish_tuning(vlt_batch* b) {
     }
     if (best >= 0) {
       t.chosen = best;
-      b->shapes[kv.first] = kCandidates[best];
+      b->shapes[kv.first] = kTileCandidates[best];
     }
   }
 }

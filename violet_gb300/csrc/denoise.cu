@@ -351,11 +351,13 @@ __device__ __forceinline__ f3 ycocg_to_rgb(f3 c) {
 // 2^-48 within 2^36, and a special code makes the clamp's bounds NaN either way.
 // 1365x767: 45 -> 30 us, 1280x720 reference frame with the clamp 595 -> 579 us.
 struct DnFastClampF {
+  // single views run 32x4 tiles, which are among the candidates of the batches
+  static constexpr int kStage = max_staged_tile(1);
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, const uint2* __restrict__ fast, uint2* __restrict__ color) {
   struct Px {
     float2 y, co, cg;  // diffuse, specular
   };
-  __shared__ Px tile[(64 + 2) * (4 + 2)];  // the largest of the tile shapes, 64x4
+  __shared__ Px tile[kStage];
   const int bx = (int)blockDim.x, by = (int)blockDim.y, pw = bx + 2;
   const int tid = (int)threadIdx.y * bx + (int)threadIdx.x;
   __syncthreads();  // a persistent block's previous tile is done with the stage

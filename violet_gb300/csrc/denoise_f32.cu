@@ -787,6 +787,10 @@ __device__ __forceinline__ void atrous_px(int x, int y, int w, int h, const Geo&
 template <class Geo, class RI, class RO, class L>
 struct Dn32AtrousF {
   static constexpr int kMinBlocks = 4;  // 64 registers (5 and 6 blocks of 256 threads spill, 2 and 3 starve)
+  // A tile's rows ascend through the image while its height divides the eight rows of a
+  // phase or is a multiple of them.
+  static constexpr bool kTileRowsFit = tile_heights_fit(8);
+  static_assert(kTileRowsFit, "tile heights");
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, AtrousDist td, const RI* __restrict__ in, RO* __restrict__ out, L* __restrict__ out_diff, L* __restrict__ out_spec, int sh) {
   // Rows are dealt out so that eight successive tile rows lie `step` apart in the image
   // (groups of 8 * step rows, within a group phase by phase): a tile's taps are then mostly
@@ -794,6 +798,8 @@ struct Dn32AtrousF {
   // the interleaved records and 32x4 tiles (32x8 was better with image rows): 3840x2160
   // f16 frame 5,808 -> 5,738 us, 320x180 f32 121 -> 118 us, 12-view f16 batch 1,385 -> 1,354 us,
   // 1920x1080 f32 unchanged (1,505). What bounds it is load latency at 32 warps per SM.
+  // `interior` takes a tile's first and last row for its lowest and highest image rows, which
+  // kTileRowsFit says they are.
   const auto row = [sh](int v) {
     const int in_group = v & ((8 << sh) - 1);
     return v - in_group + (in_group >> 3) + ((in_group & 7) << sh);

@@ -55,6 +55,34 @@ struct TileShape {
 static constexpr int kBlock1D = 128;
 static constexpr int kMaxThreads = 256;  // largest tile the autotuner tries
 
+// The batch's candidate shapes: five tile shapes, each one tile per block and persistent.
+// Every 2D pass may run in any of them.
+static constexpr TileShape kTileCandidates[VLT_TILE_CANDIDATES] = {
+    {32, 4, 0}, {16, 8, 0}, {32, 8, 0}, {16, 16, 0}, {64, 4, 0},
+    {32, 4, 1}, {16, 8, 1}, {32, 8, 1}, {16, 16, 1}, {64, 4, 1}};
+// The most pixels of a candidate tile with `halo` pixels around it, for passes that stage
+// their tile.
+constexpr int max_staged_tile(int halo) {
+  int m = 0;
+  for (const TileShape& t : kTileCandidates) {
+    const int n = (t.bx + 2 * halo) * (t.by + 2 * halo);
+    m = n > m ? n : m;
+  }
+  return m;
+}
+// Whether every candidate's height divides `rows` or is a multiple of it.
+constexpr bool tile_heights_fit(int rows) {
+  for (const TileShape& t : kTileCandidates)
+    if (rows % t.by != 0 && t.by % rows != 0) return false;
+  return true;
+}
+constexpr bool tile_threads_fit() {
+  for (const TileShape& t : kTileCandidates)
+    if (t.bx * t.by > kMaxThreads || t.bx * t.by % 32 != 0) return false;
+  return true;
+}
+static_assert(tile_threads_fit(), "blocks are whole warps of at most kMaxThreads threads");
+
 // A prepared batched launch: a kernel and its parameter block (host bytes at
 // `param_off` in the executor's parameter buffer).
 struct Prepared {
