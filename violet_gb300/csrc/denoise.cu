@@ -298,7 +298,7 @@ __device__ __forceinline__ float short_weight(const ShortPixel& c, const Geo& ge
 // written by the shader; here they get zeros.
 template <class Geo>
 struct DnFixF {
-  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
+  static constexpr int kMinBlocks = 5;  // 48 registers: most pixels only copy their record
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const uint8_t* __restrict__ len_tex, const uint2* __restrict__ color, const uint32_t* __restrict__ mom, uint2* __restrict__ out_color, uint32_t* __restrict__ out_mom) {
   __shared__ ShortStage<2> st;
   const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
@@ -417,7 +417,7 @@ struct DnFastClampF {
 // svgf_spatial_fallback_filter.hlsl:25-125. History-0 pixels get zeros.
 template <class Geo>
 struct DnFallbackF {
-  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
+  static constexpr int kMinBlocks = 5;  // 48 registers: most pixels only copy their record
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const uint8_t* __restrict__ len_tex, const uint2* __restrict__ color, const uint32_t* __restrict__ mom, uint2* __restrict__ out_color, uint32_t* __restrict__ out_var) {
   __shared__ ShortStage<3> st;
   const int x = x0 + (int)threadIdx.x, y = y0 + (int)threadIdx.y;
@@ -857,7 +857,7 @@ static void launch_atrous_tile(const Exec& ex, int w, int h, const Geo& geo, con
   const int pw = kAtrousTileX + 4 * step;
   const unsigned groups = (unsigned)((h + kAtrousTileRows * step - 1) / (kAtrousTileRows * step));
   const dim3 grid((unsigned)((w + kAtrousTileX - 1) / kAtrousTileX), groups * (unsigned)step, 1);
-  // ceil(2^32 / pw): the high word of k * pitch_inv is k / pw for k below 2^16
+  // floor(2^32 / pw) + 1: the high word of k * pitch_inv is k / pw for k below 2^16
   const uint32_t pitch_inv = (uint32_t)(((uint64_t)1 << 32) / (uint32_t)pw + 1u);
   const AtrousOut o = {(uint2*)out_color, out_var, out_diff, out_spec};
   const size_t bytes = atrous_tile_bytes(step);

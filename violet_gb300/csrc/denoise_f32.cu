@@ -435,7 +435,7 @@ __device__ __forceinline__ float short_weight(const ShortPixel& c, const Geo& ge
 
 template <class Geo, int FORM>
 struct Dn32FixF {
-  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
+  static constexpr int kMinBlocks = 5;  // 48 registers: most pixels only copy their record
   using R = typename DnT<FORM>::R;
   using N = typename DnT<FORM>::N;
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const N* __restrict__ len, const R* __restrict__ in, R* __restrict__ out) {
@@ -537,7 +537,7 @@ struct Dn32FastClampF {
 
 template <class Geo, int FORM>
 struct Dn32FallbackF {
-  static constexpr int kMinBlocks = 5;  // 51 registers: most pixels only copy their record
+  static constexpr int kMinBlocks = 5;  // 48 registers: most pixels only copy their record
   using R = typename DnT<FORM>::R;
   using N = typename DnT<FORM>::N;
   static __device__ __forceinline__ void run(int x0, int y0, int w, int h, Geo geo, const N* __restrict__ len, const R* __restrict__ in, R* __restrict__ out) {
