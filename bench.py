@@ -108,13 +108,13 @@ PASS_BYTES_PER_CELL = {"hg_decay": 2, "hg_compact": 4}
 # dram__bytes_write.sum; the a-trous from its interleaved-record launches,
 # profiles/dn_atrous_f32_540p.md; the specular spatial pass the mean of its two launches,
 # profiles/spec_spatial_f32_540p.md).
-MEASURED_TRAFFIC_PER_UNIT = {"dn_atrous": 64.1, "spec_spatial": (36.054e6 + 0.246e6 + 34.458e6 + 0.320e6) / 2 / (960 * 540)}
+MEASURED_TRAFFIC_PER_UNIT = {"dn_atrous": 64.1, "spec_spatial": (36.040e6 + 0.240e6 + 34.417e6 + 0.208e6) / 2 / (960 * 540)}
 # Warp instructions per launch unit measured with ncu (smsp__inst_executed.sum / pixels;
 # the a-trous the mean of its five launches, of which the first reads plain records): the
 # issue roofline of a pass that is bound by instruction issue or latency rather than by HBM.
 MEASURED_WARP_INSTRUCTIONS_PER_UNIT = {
     "dn_atrous": (21.536e6 + 16.045e6 + 16.055e6 + 16.126e6 + 16.056e6) / 5 / (960 * 540),
-    "spec_spatial": (39.451e6 + 43.171e6) / 2 / (960 * 540)}
+    "spec_spatial": (39.609e6 + 43.194e6) / 2 / (960 * 540)}
 ISSUE_SLOTS_PER_SM_CLOCK = 4  # one warp instruction per scheduler per clock, 4 schedulers per SM
 
 

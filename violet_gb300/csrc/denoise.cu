@@ -564,14 +564,13 @@ struct DnAtrousF {
 // frame at 1280x720 549 -> 544 us; in the float forms, which wait for loads, it gained
 // nothing).
 //
-// Bound by binary32 arithmetic: 1,834 warp instructions per 32 pixels (3,770 in the
-// per-pixel form) at 60 % issue, FMA pipe 49 % (the paired instructions take two of its
-// cycles; counted with the IEEE roots and the compared-and-rounded word codec). 1920x1080
-// from the raw G-buffer: 337 -> 121 us per iteration; from the surface
-// planes at 1280x720: 124 -> 65 us. Measured and not kept: a loop over the four tap rows
-// instead of unrolled taps (416 us for three iterations against 398), 3 or 2 blocks per SM
-// (423, 534), 16 rows by 512 threads (416), 4 rows by 128 (446), staging unrolled by two
-// (408). Above kAtrousTileMaxStep the halo outgrows the tile and the per-pixel form
+// Bound by binary32 arithmetic: 1,452 warp instructions per 32 pixels (3,770 in the
+// per-pixel form) at 67 % issue, FMA pipe 66 % (the paired instructions take two of its
+// cycles). 1920x1080 from the raw G-buffer: 337 -> 118 us per iteration; from the surface
+// planes at 1280x720: 124 -> 60 us. Measured and not kept, when three iterations took 398
+// us (356 now): a loop over the four tap rows instead of unrolled taps (416), 3 or 2 blocks
+// per SM (423, 534), 16 rows by 512 threads (416), 4 rows by 128 (446), staging unrolled by
+// two (408). Above kAtrousTileMaxStep the halo outgrows the tile and the per-pixel form
 // runs; recorded (batched) jobs, whose tile shape the batch chooses, run it too.
 constexpr int kAtrousTileMaxStep = 16;
 constexpr int kAtrousTileX = 64, kAtrousTileRows = 8;
@@ -867,8 +866,8 @@ static void launch_atrous_tile(const Exec& ex, int w, int h, const Geo& geo, con
   };
   // One output row per thread while there are few tiles per SM (a block's own latency is
   // then the pass), two rows on fewer threads for more. Five iterations, 256 / 512
-  // threads: 320x180 73 / 54 us, 640x360 134 / 114 us, 854x480 193 / 175 us; three at
-  // 1920x1080 398 / 428 us.
+  // threads: 320x180 61 / 50 us, 640x360 111 / 102 us, 854x480 163 / 156 us, 1280x720 299 /
+  // 304 us; three at 1920x1080 355 / 385 us.
   if ((int)(grid.x * grid.y) <= 8 * device_sm_count()) run(k_atrous_tile<Geo, 512>, 512);
   else run(k_atrous_tile<Geo, 256>, 256);
 }
