@@ -547,19 +547,21 @@ struct DnAtrousF {
 // pairs, and the paired binary32 instructions (one IEEE operation per component, the
 // same bits) halve the issue slots of the parts that run per channel.
 //
-// What the per-pixel form guards per tap is settled per block. The geometry is `tame`
-// when every depth is 0 or of a magnitude in [2^-70, 2^70] and no fwidth_z of the tile is
-// negative or not finite. Then the depth terms' quotients may be formed with a shared
-// reciprocal (div_shared) and no weight exponent is positive; other blocks run the
-// per-pixel form. The values are `ordinary` when every staged colour and variance is
-// finite and no variance is negative. Then the per-pixel roots and quotients are the
-// branch-free ones (three iterations at 1080p 379 -> 365 us against the IEEE operations);
-// blocks with other values take those few operations as IEEE ones, and the rest of the
-// arithmetic is the same for infinities and NaN: an overflowed variance, which the
-// iterations spread over ever more blocks (0.9 % of them in the first, 31 % in the fifth
-// in a walk at 1080p), does not take a block off the tile. An iteration at 1080p over one
-// special variance per tile, steps 1 / 4 / 16: 337 / 201 / 195 us in the per-pixel form, 148 / 136 / 160
-// so; all variances infinite at step 16: 398 (328 in the per-pixel form alone) and 210.
+// What the per-pixel form guards per tap is settled per block and pixel. The depths are
+// `tame` when every one is 0 or of a magnitude in [2^-70, 2^70]; with a fwidth_z that is
+// finite and not negative, the depth terms' quotients may be formed with a shared
+// reciprocal (div_shared) and no weight exponent is positive. Blocks of other depths and
+// pixels of other fwidth_z run the per-pixel form. The values are `ordinary` when every
+// staged colour and variance is finite and no variance is negative. Then the per-pixel
+// roots and quotients are the branch-free ones (three iterations at 1080p 379 -> 365 us
+// against the IEEE operations); blocks with other values take those few operations as IEEE
+// ones, and the rest of the arithmetic is the same for infinities and NaN: an overflowed
+// variance, which the iterations spread over ever more blocks (0.9 % of them in the first,
+// 31 % in the fifth in a walk at 1080p), does not take a block off the tile. An iteration
+// at 1080p over one special variance per tile, steps 1 / 4 / 16: 337 / 201 / 195 us in the
+// per-pixel form, 148 / 138 / 140 so; all variances infinite at step 16: 398 (328 in the
+// per-pixel form alone) and 154; all depths extreme: 441 with 256 threads, 322 with 512 (355
+// alone), so that no input is slower than without the tiles by more than the 5-8 % of step 8.
 // The normal weight's seven squarings run for two taps of a row as a pair (reference-form
 // frame at 1280x720 549 -> 544 us; in the float forms, which wait for loads, it gained
 // nothing).
@@ -574,6 +576,7 @@ struct DnAtrousF {
 // runs; recorded (batched) jobs, whose tile shape the batch chooses, run it too.
 constexpr int kAtrousTileMaxStep = 16;
 constexpr int kAtrousTileX = 64, kAtrousTileRows = 8;
+constexpr size_t kSharedPerSM = 228 * 1024, kSharedPerBlock = 1024;  // the latter reserved by the system
 
 struct AtrousPx {
   float4 a;  // diffuse.r, specular.r, diffuse.g, specular.g
@@ -604,7 +607,7 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return r;
 }
 
-// One output pixel of a block of tame geometry; s is the staged tile, li the pixel's place
+// One output pixel of a block of tame depths and ordinary fwidth_z; s is the staged tile, li the pixel's place
 // in it, pw the tile's row pitch. CHECK: the footprint may leave the image.
 template <bool CHECK, bool ORDINARY>
 __device__ __forceinline__ void atrous_tile_px(const AtrousPx* s, const float2* sv, int li, int pw, int x, int y,
@@ -731,12 +734,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
   // Tile rows: blockIdx.y counts (group of 8 * step image rows, phase within it).
   const int group = (int)blockIdx.y / step, phase = (int)blockIdx.y - group * step;
   const int x0 = (int)blockIdx.x * kAtrousTileX, y0 = group * (kAtrousTileRows * step) + phase;
-  uint32_t odd = 0u;  // 1: a value, 2: the geometry
+  uint32_t odd = 0u;  // 1: a value, 2: a depth
   const auto tame_depth = [](float d) { return d == 0.0f || (fabsf(d) >= 0x1p-70f && fabsf(d) <= 0x1p70f); };
-  const auto tame_fwz = [](float f) { return f >= 0.0f && f < 1e6f; };
-  const auto in_tile = [=](int row, int col) {
-    return row >= 2 && row < kAtrousTileRows + 2 && col >= 2 * step && col < kAtrousTileX + 2 * step;
-  };
   for (int k = tid; k < np; k += NT) {
     const int row = (int)__umulhi((uint32_t)k, pitch_inv), col = k - row * pw;  // k / pw (host: exact for k < np)
     const int gx = x0 + col - 2 * step, gy = y0 + (row - 2) * step;
@@ -757,7 +756,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
     // a luminance is finite where its channels are
     if (!(px.b.z < 1e6f && px.b.w < 1e6f && v.x >= 0.0f && v.y >= 0.0f && v.x < 1e6f && v.y < 1e6f)) odd |= 1u;
     if (!tame_depth(dep)) odd |= 2u;
-    if (in_tile(row, col) && !tame_fwz(geo.fwz(i))) odd |= 2u;
   }
   const bool ordinary = __syncthreads_and(odd == 0u);
   const bool tame = ordinary || __syncthreads_and(odd < 2u);
@@ -769,11 +767,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT)  // 64 registers
   for (int row = ty; row < kAtrousTileRows; row += NT / kAtrousTileX) {
     const int x = x0 + tx, y = y0 + row * step;
     if (!inb(x, y, w, h)) return;
-    if (!tame) {
+    const float fwz = geo.fwz((size_t)y * w + x);
+    if (!(tame && fwz >= 0.0f && fwz < 1e6f)) {
       atrous_px(x, y, w, h, geo, taps, color, var_tex, o.color, o.var, o.diff, o.spec, step);
       continue;
     }
-    const float fwz = geo.fwz((size_t)y * w + x);
     const int li = (row + 2) * pw + tx + 2 * step;
     if (!ordinary) atrous_tile_px<true, false>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
     else if (interior) atrous_tile_px<false, true>(s, sv, li, pw, x, y, w, h, fwz, td, step, o, one);
@@ -868,7 +866,11 @@ static void launch_atrous_tile(const Exec& ex, int w, int h, const Geo& geo, con
   // then the pass), two rows on fewer threads for more. Five iterations, 256 / 512
   // threads: 320x180 61 / 50 us, 640x360 111 / 102 us, 854x480 163 / 156 us, 1280x720 299 /
   // 304 us; three at 1920x1080 355 / 385 us.
-  if ((int)(grid.x * grid.y) <= 8 * device_sm_count()) run(k_atrous_tile<Geo, 512>, 512);
+  // One row per thread also where shared memory leaves room for two blocks per SM only
+  // (steps above 12): 256 threads are then 16 warps, and step 16 at 1920x1080 takes 152 us
+  // instead of 135 (at step 8, where three blocks fit, 125 instead of 129).
+  if ((int)(grid.x * grid.y) <= 8 * device_sm_count() || 3 * (bytes + kSharedPerBlock) > kSharedPerSM)
+    run(k_atrous_tile<Geo, 512>, 512);
   else run(k_atrous_tile<Geo, 256>, 256);
 }
 
